@@ -25,6 +25,7 @@ SOURCES = [  # (file, extra flags)
     ('dsum.cu', ['-fmad=false']),
     ('mesh.cu', ['-fmad=false', '-Xcompiler', '-fopenmp']),
     ('tiles.cu', ['-fmad=false']),
+    ('fast_tiles.cu', ['-fmad=false']),
     ('batch.cu', ['-fmad=false']),
     ('batch_mixed.cu', ['-fmad=true']),     # the mixed form: fused multiply-adds allowed
 ]

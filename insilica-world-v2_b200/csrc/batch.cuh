@@ -11,16 +11,16 @@ namespace isw {
 namespace bt {
 
 constexpr int FAST_KMAX = 8;                  // the largest exchange interval of the tiled fast loop
-constexpr int FAST_CMAX = 4;                  // mixed tiles: cells per thread at most (nc <= FAST_CMAX x threads)
-constexpr int FAST_EMAX = 8;                  // mixed tiles: edges per thread at most
-constexpr int FAST_AMAX = 4;                  // mixed tiles: owned edges per thread at most (their sums in registers)
 
 struct TileSetDev {
   int P, k;
-  const int *cell_off, *edge_off, *cells, *edges, *ncnt, *ecnt, *eown;
-  const int16_t *cedge, *eIl, *eJl;
-  const double *ade, *ale, *aarea;            // d_e, l_e per local edge and the area per local cell, in local order
-  const float *arde32, *ale32, *arA32;        // the mixed form's: 1 / d_e, l_e, 1 / area, in local order
+  const int *cell_off, *edge_off, *ncnt, *ecnt, *eown, *nbr_off, *nbrs;
+  const uint4 *cedge, *casc;
+  const int2 *eix;
+  const double2 *el;                          // (l_e, d_e) per local edge
+  const float2 *el32;                         // the mixed form's (l_e, 1 / d_e)
+  const double *aarea;                        // the area per local cell
+  const float *arA32;                         // and its FP32 reciprocal
 };
 
 struct StackDesc {
@@ -35,6 +35,7 @@ struct StackDesc {
   int n[3];
   double cdt[3], tau[3], inv_n[3];
   TileSetDev tiles;
+  int tile_base;             // the stack's first tile in the batch's list (and its first flag)
 };
 
 struct Chunk {
@@ -64,8 +65,8 @@ __device__ __forceinline__ void raise_status(BatchStatus *s, int code) {
 struct Sched {
   const Chunk *cell, *edge, *vert, *rows, *erows;   // rows: (tracer, cell) pairs; erows: (tracer, edge) pairs
   int ncell, nedge, nvert, nrows, nerows;
-  const Chunk *wcell, *wedge;                       // the same in the sub-step passes' chunks (SUB_W... x THREADS)
-  int nwcell, nwedge;
+  const Chunk *wcell, *wedge, *uedge;               // untiled stacks only: the sub-step passes' chunks (SUB_W... x THREADS),
+  int nwcell, nwedge, nuedge;                       // and their edges in plain chunks
   BatchStatus *status;
 };
 
@@ -169,10 +170,10 @@ __device__ __forceinline__ const StackDesc &stage_desc(const StackDesc *S, int s
 // P2E (stage-2 fluxes), P2 (cells: p2), P3E (antidiffusive fluxes), P3 (cells: ratios), P4 (cells: limited update).
 // A pipelined batch splits POST into VMIX (edges, the dynamics' last pass) and HF1 ((tracer, edge), the transport's first);
 // a batch with air stacks runs VMIX, VHEAT (cells: the stress's heat back to theta) and HF1 in place of POST.
-// PH_UF / PH_CS: the grid-wide edge sub-step that also forms the layer fluxes on a stack's last sub-step, and phase C
-// summing them; used by batches with no tiled stack in place of PH_U / PH_C.
-enum Phase { PH_INIT, PH_LAPE1, PH_LAPCV, PH_LAPE2, PH_A, PH_E, PH_S, PH_ETA, PH_U, PH_C, PH_D, PH_POST, PH_P2, PH_P3, PH_P4,
-             PH_P1, PH_P2E, PH_P3E, PH_VMIX, PH_HF1, PH_UF, PH_CS, PH_VHEAT, PH_ONBED };
+// PH_ETA / PH_UF: the grid-wide cell and edge sub-steps of the untiled stacks (UF also forms the layer fluxes on a stack's
+// last sub-step); PH_CS and PH_D: their limiter and their stage's end (tiled stacks end their stage in the tile kernel).
+enum Phase { PH_INIT, PH_LAPE1, PH_LAPCV, PH_LAPE2, PH_A, PH_E, PH_S, PH_ETA, PH_UF, PH_CS, PH_D, PH_POST, PH_P2, PH_P3, PH_P4,
+             PH_P1, PH_P2E, PH_P3E, PH_VMIX, PH_HF1, PH_VHEAT, PH_ONBED };
 
 // Programmatic dependent launch between phase kernels: a phase kernel is launched while the previous one drains; it
 // stages only constant data (its stack descriptor) before waiting for the previous grid's completion and memory
@@ -198,21 +199,27 @@ void launch_phase_kernel(void (*kern)(KA...), int nb, cudaStream_t st, bool pdl,
 // Domains of a phase, in block order: which chunk tables its blocks walk.
 template <int PH>
 struct Dom {
-  static constexpr bool cell = PH == PH_INIT || PH == PH_LAPCV || PH == PH_A || PH == PH_ETA || PH == PH_C || PH == PH_D ||
-                               PH == PH_CS || PH == PH_VHEAT || PH == PH_ONBED;
-  static constexpr bool edge = PH == PH_INIT || PH == PH_LAPE1 || PH == PH_LAPE2 || PH == PH_E || PH == PH_S || PH == PH_U ||
-                               PH == PH_D || PH == PH_POST || PH == PH_VMIX || PH == PH_UF;
+  static constexpr bool cell = PH == PH_INIT || PH == PH_LAPCV || PH == PH_A || PH == PH_ETA || PH == PH_D || PH == PH_CS ||
+                               PH == PH_VHEAT || PH == PH_ONBED;
+  static constexpr bool edge = PH == PH_INIT || PH == PH_LAPE1 || PH == PH_LAPE2 || PH == PH_E || PH == PH_S || PH == PH_D ||
+                               PH == PH_POST || PH == PH_VMIX || PH == PH_UF;
   static constexpr bool vert = PH == PH_INIT || PH == PH_LAPCV || PH == PH_A;
   static constexpr bool rows = PH == PH_P1 || PH == PH_P2 || PH == PH_P3 || PH == PH_P4;
   static constexpr bool erows = PH == PH_POST || PH == PH_P2E || PH == PH_P3E || PH == PH_HF1;
-  static constexpr bool wide = PH == PH_ETA || PH == PH_U || PH == PH_UF;   // cells / edges in the wide chunks
+  static constexpr bool wide = PH == PH_ETA || PH == PH_UF;                    // cells / edges in the wide chunks
+  static constexpr bool untiled = wide || PH == PH_CS || PH == PH_D;           // of the untiled stacks only
 };
+static_assert(SUB_WC == 1, "the untiled stacks' wide cell chunks are also their plain ones");
+
+template <int PH>
+__host__ __device__ inline int cell_chunks(const Sched &sc) { return Dom<PH>::untiled ? sc.nwcell : sc.ncell; }
+template <int PH>
+__host__ __device__ inline int edge_chunks(const Sched &sc) { return Dom<PH>::wide ? sc.nwedge : Dom<PH>::untiled ? sc.nuedge : sc.nedge; }
 
 // Blocks of a phase over a schedule.
 template <int PH>
 inline int phase_blocks(const Sched &sc) {
-  return (Dom<PH>::cell ? (Dom<PH>::wide ? sc.nwcell : sc.ncell) : 0) +
-         (Dom<PH>::edge ? (Dom<PH>::wide ? sc.nwedge : sc.nedge) : 0) + (Dom<PH>::vert ? sc.nvert : 0) +
+  return (Dom<PH>::cell ? cell_chunks<PH>(sc) : 0) + (Dom<PH>::edge ? edge_chunks<PH>(sc) : 0) + (Dom<PH>::vert ? sc.nvert : 0) +
          (Dom<PH>::rows ? sc.nrows : 0) + (Dom<PH>::erows ? sc.nerows : 0);
 }
 
@@ -220,13 +227,13 @@ inline int phase_blocks(const Sched &sc) {
 template <int PH>
 __device__ __forceinline__ int phase_chunk(const Sched &sc, int b, Chunk &ch) {
   if (Dom<PH>::cell) {
-    const int n = Dom<PH>::wide ? sc.nwcell : sc.ncell;
-    if (b < n) { ch = (Dom<PH>::wide ? sc.wcell : sc.cell)[b]; return 0; }
+    const int n = cell_chunks<PH>(sc);
+    if (b < n) { ch = (Dom<PH>::untiled ? sc.wcell : sc.cell)[b]; return 0; }
     b -= n;
   }
   if (Dom<PH>::edge) {
-    const int n = Dom<PH>::wide ? sc.nwedge : sc.nedge;
-    if (b < n) { ch = (Dom<PH>::wide ? sc.wedge : sc.edge)[b]; return 1; }
+    const int n = edge_chunks<PH>(sc);
+    if (b < n) { ch = (Dom<PH>::wide ? sc.wedge : Dom<PH>::untiled ? sc.uedge : sc.edge)[b]; return 1; }
     b -= n;
   }
   if (Dom<PH>::vert) { if (b < sc.nvert) { ch = sc.vert[b]; return 2; } b -= sc.nvert; }
@@ -241,12 +248,15 @@ constexpr size_t S_STAGE_MAX = 64 * 1024;   // the slow tendency's staged neighb
 void launch_phase_mixed(int ph, int lmax, int nb, cudaStream_t st, bool pdl, size_t smem, const StackDesc *desc,
                         const Sched &sc, int stage, int j);
 void slow_phase_smem_mixed(size_t bytes);
-const void *fast_kernel_mixed(int bps);
 const void *fast_grid_kernel_mixed();
 void launch_fast_grid_mixed(const cudaLaunchConfig_t &cfg, const StackDesc *desc, const Sched &sc, int stage, int nsub,
-                            int flux, GridBarrier *bar, BatchStatus *status, long long timeout_ns);
-void launch_fast_mixed(int bps, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage, int rounds,
-                       GridBarrier *bar, BatchStatus *status, long long timeout_ns, int fault_block);
+                            GridBarrier *bar, BatchStatus *status, long long timeout_ns);
+
+// The tiled fast loop (fast_tiles.cu): a form's kernel for `bps` tile blocks per SM, its block size, and its launch.
+const void *fast_tiles_kernel(int bps, bool mixed);
+int fast_tiles_threads(int bps);
+void launch_fast_tiles(int bps, bool mixed, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
+                       unsigned *flags, BatchStatus *status, long long timeout_ns, int fault_block);
 
 }  // namespace bt
 }  // namespace isw

@@ -1,39 +1,19 @@
 // The batched step's kernels for stacks in the mixed form (layers_mixed.cuh, transport_mixed.cuh): the same phase list,
 // chunk tables and tiles as the plain FP64 kernels in batch.cu, compiled with fused multiply-adds (this file alone).
-// The tile kernel runs the fast loop in deviation form (deta, dub in FP32, their FP64 sum acc) in shared memory.
 #include "batch.cuh"
 #include "layers_mixed.cuh"
+#include "mixed_stage.cuh"
 #include "transport_mixed.cuh"
 
 namespace isw {
 namespace bt {
 namespace {
 
-__device__ __forceinline__ mixed::MStageArgs mstage_args(const StackDesc &d, int st) {
-  const LayersDev &M = d.M;
-  mixed::MStageArgs a;
-  a.h0 = d.h;
-  a.u0 = d.u;
-  a.u0f = M.u32;
-  a.hs = st == 0 ? d.h : st == 1 ? M.h1 : M.h2;
-  a.us = st == 0 ? M.u32 : st == 1 ? M.u1f : M.u2f;
-  a.hn = st == 0 ? M.h1 : st == 1 ? M.h2 : d.h;
-  a.un = st == 2 ? d.u : nullptr;
-  a.unf = st == 0 ? M.u1f : st == 1 ? M.u2f : nullptr;
-  a.Fm = st == 2 ? d.Fm : nullptr;
-  a.cdt = d.cdt[st];
-  a.dt = d.dt;
-  a.tau = (float)d.tau[st];
-  a.inv_n = d.inv_n[st];
-  a.n = d.n[st];
-  return a;
-}
-
 // The grid-wide sub-step passes over a wide chunk: PH_ETA's cells (sub-step 0 item by item, as it also forms the slot
-// coefficients), PH_U's / PH_UF's edges (PH_UF also forming the layer fluxes on the stack's last sub-step).
+// coefficients), PH_UF's edges (also forming the layer fluxes on the stack's last sub-step).
 template <int PH>
 __device__ __forceinline__ void substep_chunk(const StackDesc &d, int st, int j, const Chunk &ch) {
-  if (d.tiled || j >= d.n[st]) return;
+  if (j >= d.n[st]) return;
   const LayersDev &M = d.M;
   const float tau = (float)d.tau[st];
   const int first = ch.begin + (int)threadIdx.x;
@@ -44,8 +24,8 @@ __device__ __forceinline__ void substep_chunk(const StackDesc &d, int st, int j,
       mixed::bt_eta_cells<SUB_WC>(M, tau, j, d.n[st], first, ch.end);
   } else {
     mixed::bt_u_edges(M, tau, j, d.n[st], first, ch.end);
-    if (PH == PH_UF && j == d.n[st] - 1) {
-      const mixed::MStageArgs a = mstage_args(d, st);
+    if (j == d.n[st] - 1) {
+      const mixed::MStageArgs a = mixed::mstage_args(d, st);
       for (int i = first; i < ch.end; i += THREADS) mixed::flux_edge(M, a, M.acc[i], i);
     }
   }
@@ -66,7 +46,7 @@ __global__ void __launch_bounds__(THREADS) k_phase_m(const StackDesc *__restrict
   const int i = ch.begin + (int)threadIdx.x;
   if (PH == PH_S && d.s_stage) {             // the block stages its rows' distinct neighbour records, then computes
     extern __shared__ __align__(16) float4 stg4[];
-    const mixed::MStageArgs a = mstage_args(d, st);
+    const mixed::MStageArgs a = mixed::mstage_args(d, st);
     ISW_BATCH_L(d.L, LMAXK, mixed::stage_pk4<LL>(d.M, ch.begin / THREADS, stg4));
     __syncthreads();
     if (i < ch.end) ISW_BATCH_L(d.L, LMAXK, (mixed::slow_edge<LL, true>(d.M, a.us, a.cdt, i, stg4)));
@@ -91,23 +71,20 @@ __global__ void __launch_bounds__(THREADS) k_phase_m(const StackDesc *__restrict
       else ISW_BATCH_L(d.L, LMAXK, (mixed::curl_vertex<LL, float>(M, M.L1f, i)));
     }
   } else if (PH == PH_A) {
-    const mixed::MStageArgs a = mstage_args(d, st);
+    const mixed::MStageArgs a = mixed::mstage_args(d, st);
     if (kind == 0) ISW_BATCH_L(d.L, LMAXK, mixed::bern_cell<LL>(M, a.hs, a.us, i));
     else ISW_BATCH_L(d.L, LMAXK, mixed::pv_vertex<LL>(M, a.hs, a.us, i));
   } else if (PH == PH_E) {
-    const mixed::MStageArgs a = mstage_args(d, st);
+    const mixed::MStageArgs a = mixed::mstage_args(d, st);
     ISW_BATCH_L(d.L, LMAXK, mixed::edge_hq<LL>(M, a.hs, a.us, i));
   } else if (PH == PH_S) {
-    const mixed::MStageArgs a = mstage_args(d, st);
+    const mixed::MStageArgs a = mixed::mstage_args(d, st);
     ISW_BATCH_L(d.L, LMAXK, mixed::slow_edge<LL>(M, a.us, a.cdt, i));
-  } else if (PH == PH_C) {
-    const mixed::MStageArgs a = mstage_args(d, st);
-    ISW_BATCH_L(d.L, LMAXK, mixed::scale_cell<LL>(M, a, i));
   } else if (PH == PH_CS) {
-    const mixed::MStageArgs a = mstage_args(d, st);
+    const mixed::MStageArgs a = mixed::mstage_args(d, st);
     ISW_BATCH_L(d.L, LMAXK, mixed::scale_sum_cell<LL>(M, a, i));
   } else if (PH == PH_D) {
-    const mixed::MStageArgs a = mstage_args(d, st);
+    const mixed::MStageArgs a = mixed::mstage_args(d, st);
     if (kind == 0) {
       ISW_BATCH_L(d.L, LMAXK, mixed::h_cell<LL>(M, a, i));
       if (st == 2) check_finite_column(d.h, M.g.N, d.L, i, sc.status);
@@ -142,162 +119,6 @@ __global__ void __launch_bounds__(THREADS) k_phase_m(const StackDesc *__restrict
   }
 }
 
-// The fast loop of stage `st` over every tiled stack in the mixed form (the tile scheme of batch.cu's k_fast). Shared
-// memory, FP32 arrays: per cell deta, Y = Gc (deta + gamma (deta - deta_prev)), 1/area, Gc, c0 = sum sign l_e H_e ubar0
-// and its 8 edge slots (16 bytes); per edge dub, fl = l_e H_e dub (what the cell pass sums: one float per gathered
-// edge), l_e H_e, G', 1/d_e and its two local cells. A thread's edges are always e = tid + j NT, so the FP64 sub-step
-// sum acc of its owned edges (j < FAST_AMAX) stays in registers. Exchange buffers xeta[r & 1] and xdub[r & 1]; the
-// final dub and acc go to dub and acc, which no round reads. The host keeps nc <= FAST_CMAX NT, ne <= FAST_EMAX NT and
-// eown <= FAST_AMAX NT.
-template <int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_fast_m(const StackDesc *__restrict__ S, const TileRef *__restrict__ refs, int st,
-                                                      int rounds, GridBarrier *bar, BatchStatus *status, long long timeout_ns,
-                                                      int fault_block) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int cnt[2 * (FAST_KMAX + 1)];
-  const TileRef tr = refs[blockIdx.x];
-  const StackDesc &d = S[tr.s];
-  const LayersDev &M = d.M;
-  const TileSetDev &T = d.tiles;
-  const int p = tr.p, k = T.k;
-  const int c0i = T.cell_off[p], nc = T.cell_off[p + 1] - c0i;
-  const int e0 = T.edge_off[p], ne = T.edge_off[p + 1] - e0;
-  const int eown = T.eown[p];
-  const int *cells = T.cells + c0i;
-  const int *edges = T.edges + e0;
-  uint4 *cedge = reinterpret_cast<uint4 *>(smem);
-  float *deta = reinterpret_cast<float *>(cedge + nc);
-  float *Y = deta + nc;
-  float *rA = Y + nc;
-  float *gc = rA + nc;
-  float *cz = gc + nc;
-  float *dub = cz + nc;
-  float *fl = dub + ne;
-  float *lh = fl + ne;
-  float *G = lh + ne;
-  float *rde = G + ne;
-  short2 *eij = reinterpret_cast<short2 *>(rde + ne);
-  const int skip = (int)blockIdx.x == fault_block;
-  const int n = d.n[st];
-  const float tau = (float)d.tau[st], gam = (float)M.div_damp;
-  const int t = threadIdx.x;
-  if (t <= k) {
-    cnt[t] = T.ncnt[(size_t)p * (k + 1) + t];
-    cnt[FAST_KMAX + 1 + t] = T.ecnt[(size_t)p * (k + 1) + t];
-  }
-  double accr[FAST_AMAX];
-#pragma unroll
-  for (int j = 0; j < FAST_AMAX; j++) accr[j] = 0.0;
-  const uint4 *gcedge = reinterpret_cast<const uint4 *>(T.cedge) + c0i;
-  for (int c = t; c < nc; c += NT) {
-    deta[c] = 0.f;
-    rA[c] = T.arA32[c0i + c];
-    gc[c] = M.Gc32[cells[c]];
-    cedge[c] = gcedge[c];
-  }
-  for (int e = t; e < ne; e += NT) {
-    const int ge = edges[e];
-    const float l = T.ale32[e0 + e] * M.He32[ge];
-    lh[e] = l;
-    fl[e] = l * (float)M.ub0[ge];          // ubar0's flux for the c0 pass below, then zero
-    G[e] = M.G32[ge];
-    rde[e] = T.arde32[e0 + e];
-    eij[e] = make_short2(T.eIl[e0 + e], T.eJl[e0 + e]);
-  }
-  __syncthreads();
-  for (int c = t; c < nc; c += NT) {
-    const uint4 w = cedge[c];
-    const int vs[6] = {(int16_t)(w.x & 0xffff), (int16_t)(w.x >> 16), (int16_t)(w.y & 0xffff), (int16_t)(w.y >> 16),
-                       (int16_t)(w.z & 0xffff), (int16_t)(w.z >> 16)};
-    float s = 0.f;
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-      const int v = vs[q];
-      if (v == 0) continue;
-      const float f = fl[(v > 0 ? v : -v) - 1];
-      s += v > 0 ? f : -f;
-    }
-    cz[c] = s;
-  }
-  __syncthreads();
-  for (int e = t; e < ne; e += NT) {
-    dub[e] = 0.f;
-    fl[e] = 0.f;
-  }
-  const int nown = cnt[0];
-  for (int r = 0; r < rounds; r++) {
-    const int K = min(k, n - r * k);
-    if (r > 0) {
-      if (!grid_sync(bar, status, timeout_ns, skip)) return;
-      if (K > 0) {
-        const float *xe = M.xeta[(r - 1) & 1];
-        const float *xu = M.xdub[(r - 1) & 1];
-        for (int c = nown + t; c < nc; c += NT) deta[c] = xe[cells[c]];
-        for (int e = eown + t; e < ne; e += NT) {
-          const float v = xu[edges[e]];
-          dub[e] = v;
-          fl[e] = lh[e] * v;
-        }
-      }
-    }
-    __syncthreads();
-    for (int m = 1; m <= K; m++) {
-      const int cn = cnt[K - m + 1];
-#pragma unroll
-      for (int j = 0; j < FAST_CMAX; j++) {
-        const int c = t + j * NT;
-        if (c < cn) {
-          const float d0 = deta[c];
-          const uint4 w = cedge[c];
-          const int vs[6] = {(int16_t)(w.x & 0xffff), (int16_t)(w.x >> 16), (int16_t)(w.y & 0xffff), (int16_t)(w.y >> 16),
-                             (int16_t)(w.z & 0xffff), (int16_t)(w.z >> 16)};
-          float div = cz[c];
-#pragma unroll
-          for (int q = 0; q < 6; q++) {
-            const int v = vs[q];
-            if (v == 0) continue;
-            const float f = fl[(v > 0 ? v : -v) - 1];
-            div += v > 0 ? f : -f;
-          }
-          const float dn = d0 - tau * div * rA[c];
-          deta[c] = dn;
-          Y[c] = gc[c] * (dn + gam * (dn - d0));
-        }
-      }
-      __syncthreads();
-      const int en = cnt[FAST_KMAX + 1 + K - m];
-#pragma unroll
-      for (int j = 0; j < FAST_EMAX; j++) {
-        const int e = t + j * NT;
-        if (e < en) {
-          const float v = dub[e];
-          const short2 ij = eij[e];
-          if (j < FAST_AMAX && e < eown) accr[j < FAST_AMAX ? j : 0] += (double)v;
-          const float nv = v + tau * (G[e] - (Y[ij.y] - Y[ij.x]) * rde[e]);
-          dub[e] = nv;
-          fl[e] = lh[e] * nv;
-        }
-      }
-      __syncthreads();
-    }
-    if (r + 1 < rounds && K > 0) {
-      float *xe = M.xeta[r & 1];
-      float *xu = M.xdub[r & 1];
-      for (int c = t; c < nown; c += NT) xe[cells[c]] = deta[c];
-      for (int e = t; e < eown; e += NT) xu[edges[e]] = dub[e];
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < FAST_AMAX; j++) {
-    const int e = t + j * NT;
-    if (e < eown) {
-      M.dub[edges[e]] = dub[e];
-      M.acc[edges[e]] = accr[j];
-    }
-  }
-}
-
 template <int PH>
 void launch_m(int lmax, int nb, cudaStream_t st, bool pdl, size_t smem, const StackDesc *desc, const Sched &sc, int stage,
               int j) {
@@ -328,8 +149,6 @@ void launch_phase_mixed(int ph, int lmax, int nb, cudaStream_t st, bool pdl, siz
     case PH_E: launch_m<PH_E>(lmax, nb, st, pdl, smem, desc, sc, stage, j); break;
     case PH_S: launch_m<PH_S>(lmax, nb, st, pdl, smem, desc, sc, stage, j); break;
     case PH_ETA: launch_m<PH_ETA>(lmax, nb, st, pdl, smem, desc, sc, stage, j); break;
-    case PH_U: launch_m<PH_U>(lmax, nb, st, pdl, smem, desc, sc, stage, j); break;
-    case PH_C: launch_m<PH_C>(lmax, nb, st, pdl, smem, desc, sc, stage, j); break;
     case PH_UF: launch_m<PH_UF>(lmax, nb, st, pdl, smem, desc, sc, stage, j); break;
     case PH_CS: launch_m<PH_CS>(lmax, nb, st, pdl, smem, desc, sc, stage, j); break;
     case PH_D: launch_m<PH_D>(lmax, nb, st, pdl, smem, desc, sc, stage, j); break;
@@ -349,9 +168,9 @@ void launch_phase_mixed(int ph, int lmax, int nb, cudaStream_t st, bool pdl, siz
 namespace {
 
 // The grid-wide fast loop of stage `st` for the untiled mixed stacks as one cooperative launch (batch.cu's k_fast_grid
-// with the mixed form's per-item arithmetic: PH_ETA's and PH_U's / PH_UF's of k_phase_m).
+// with the mixed form's per-item arithmetic: PH_ETA's and PH_UF's of k_phase_m).
 __global__ void __launch_bounds__(THREADS) k_fast_grid_m(const StackDesc *__restrict__ S, const Sched sc, int st, int nsub,
-                                                          int flux, GridBarrier *bar, BatchStatus *status, long long timeout_ns) {
+                                                          GridBarrier *bar, BatchStatus *status, long long timeout_ns) {
   __shared__ __align__(16) unsigned char buf[sizeof(StackDesc)];
   const StackDesc &d = *reinterpret_cast<const StackDesc *>(buf);
   int cur = -1;
@@ -365,20 +184,20 @@ __global__ void __launch_bounds__(THREADS) k_fast_grid_m(const StackDesc *__rest
     cur = s;
   };
   for (int j = 0; j < nsub; j++) {
-    for (int c = blockIdx.x; c < sc.ncell; c += gridDim.x) {
-      const Chunk ch = sc.cell[c];
+    for (int c = blockIdx.x; c < sc.nwcell; c += gridDim.x) {
+      const Chunk ch = sc.wcell[c];
       select(ch.s);
       const int i = ch.begin + (int)threadIdx.x;
-      if (i < ch.end && !d.tiled && j < d.n[st]) mixed::bt_eta_cell(d.M, (float)d.tau[st], j, d.n[st], i);
+      if (i < ch.end && j < d.n[st]) mixed::bt_eta_cell(d.M, (float)d.tau[st], j, d.n[st], i);
     }
     if (!grid_sync(bar, status, timeout_ns, 0)) return;
-    for (int c = blockIdx.x; c < sc.nedge; c += gridDim.x) {
-      const Chunk ch = sc.edge[c];
+    for (int c = blockIdx.x; c < sc.nuedge; c += gridDim.x) {
+      const Chunk ch = sc.uedge[c];
       select(ch.s);
       const int i = ch.begin + (int)threadIdx.x;
-      if (i < ch.end && !d.tiled && j < d.n[st]) {
+      if (i < ch.end && j < d.n[st]) {
         mixed::bt_u_edge(d.M, (float)d.tau[st], j, d.n[st], i);
-        if (flux && j == d.n[st] - 1) mixed::flux_edge(d.M, mstage_args(d, st), d.M.acc[i], i);
+        if (j == d.n[st] - 1) mixed::flux_edge(d.M, mixed::mstage_args(d, st), d.M.acc[i], i);
       }
     }
     if (!grid_sync(bar, status, timeout_ns, 0)) return;
@@ -390,20 +209,8 @@ __global__ void __launch_bounds__(THREADS) k_fast_grid_m(const StackDesc *__rest
 const void *fast_grid_kernel_mixed() { return (const void *)k_fast_grid_m; }
 
 void launch_fast_grid_mixed(const cudaLaunchConfig_t &cfg, const StackDesc *desc, const Sched &sc, int stage, int nsub,
-                            int flux, GridBarrier *bar, BatchStatus *status, long long timeout_ns) {
-  ISW_CUDA(cudaLaunchKernelEx(&cfg, k_fast_grid_m, desc, sc, stage, nsub, flux, bar, status, timeout_ns));
-}
-
-const void *fast_kernel_mixed(int bps) {
-  return bps == 2 ? (const void *)k_fast_m<512, 2> : (const void *)k_fast_m<1024, 1>;
-}
-
-void launch_fast_mixed(int bps, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage, int rounds,
-                       GridBarrier *bar, BatchStatus *status, long long timeout_ns, int fault_block) {
-  if (bps == 2)
-    ISW_CUDA(cudaLaunchKernelEx(&cfg, k_fast_m<512, 2>, desc, refs, stage, rounds, bar, status, timeout_ns, fault_block));
-  else
-    ISW_CUDA(cudaLaunchKernelEx(&cfg, k_fast_m<1024, 1>, desc, refs, stage, rounds, bar, status, timeout_ns, fault_block));
+                            GridBarrier *bar, BatchStatus *status, long long timeout_ns) {
+  ISW_CUDA(cudaLaunchKernelEx(&cfg, k_fast_grid_m, desc, sc, stage, nsub, bar, status, timeout_ns));
 }
 
 }  // namespace bt

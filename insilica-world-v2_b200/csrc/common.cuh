@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stddef.h>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -193,4 +195,6 @@ struct isw_grid {
   std::vector<int32_t> h_nbr, h_cellEdge, h_eI, h_eJ;   // host copies the fast-loop tiles are built from
   std::vector<int8_t> h_cellSign;
   std::vector<double> h_de, h_le, h_areaCell;
+  std::mutex tile_mu;                                   // guards tile_store: the grid's tile sets, shared by its batches
+  std::shared_ptr<void> tile_store;                     // (batch.cu's TileStore, made on first use)
 };

@@ -174,8 +174,9 @@ class Member:
         n = sum(max(1, int(np.ceil(c * self.stacks[0].nfast))) for c in (1 / 3, 1 / 2, 1.0))
         nu4 = any(s.core.nu4 for s in self.stacks)
         tr = any(s.T for s in self.stacks)
-        fast = 3 * info['groups'] if info['tiles'] else (3 if info['persistent'] else 2 * n)
-        return 1 + (3 if nu4 else 0) + 3 * 5 + fast + 1 + (6 if tr else 0)
+        # per stage A, E, S, then the tile launches, or the grid-wide sub-steps with the limiter and the stage's end
+        fast = 3 * info['groups'] if info['tiles'] else (3 if info['persistent'] else 2 * n) + 3 * 2
+        return 1 + (3 if nu4 else 0) + 3 * 3 + fast + 1 + (6 if tr else 0)
 
 
 def _fp64_kinds(dg, fp64_kinds):
