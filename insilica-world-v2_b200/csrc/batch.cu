@@ -901,17 +901,17 @@ void launch_phase(isw_batch *b, cudaStream_t st, int stage, int j, bool pdl = tr
     const size_t smem = PH == PH_S ? b->s_smem[0] : 0;
     if (b->any_ext) {
       switch (b->lmax) {
-        case 2: launch_phase_kernel(k_phase<PH, 2, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        case 3: launch_phase_kernel(k_phase<PH, 3, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        case 5: launch_phase_kernel(k_phase<PH, 5, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        default: launch_phase_kernel(k_phase<PH, 8, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
+        case 2: launch_kernel(k_phase<PH, 2, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
+        case 3: launch_kernel(k_phase<PH, 3, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
+        case 5: launch_kernel(k_phase<PH, 5, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
+        default: launch_kernel(k_phase<PH, 8, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
       }
     } else {
       switch (b->lmax) {
-        case 2: launch_phase_kernel(k_phase<PH, 2, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        case 3: launch_phase_kernel(k_phase<PH, 3, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        case 5: launch_phase_kernel(k_phase<PH, 5, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        default: launch_phase_kernel(k_phase<PH, 8, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
+        case 2: launch_kernel(k_phase<PH, 2, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
+        case 3: launch_kernel(k_phase<PH, 3, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
+        case 5: launch_kernel(k_phase<PH, 5, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
+        default: launch_kernel(k_phase<PH, 8, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
       }
     }
   }

@@ -175,27 +175,6 @@ __device__ __forceinline__ const StackDesc &stage_desc(const StackDesc *S, int s
 enum Phase { PH_INIT, PH_LAPE1, PH_LAPCV, PH_LAPE2, PH_A, PH_E, PH_S, PH_ETA, PH_UF, PH_CS, PH_D, PH_POST, PH_P2, PH_P3, PH_P4,
              PH_P1, PH_P2E, PH_P3E, PH_VMIX, PH_HF1, PH_VHEAT, PH_ONBED };
 
-// Programmatic dependent launch between phase kernels: a phase kernel is launched while the previous one drains; it
-// stages only constant data (its stack descriptor) before waiting for the previous grid's completion and memory
-// (griddepcontrol.wait), and lets its own dependent launch at once (griddepcontrol.launch_dependents).
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <class... KA, class... A>
-void launch_phase_kernel(void (*kern)(KA...), int nb, cudaStream_t st, bool pdl, size_t smem, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)nb);
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl ? 1 : 0;
-  ISW_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
-}
-
 // Domains of a phase, in block order: which chunk tables its blocks walk.
 template <int PH>
 struct Dom {

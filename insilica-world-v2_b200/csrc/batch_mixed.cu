@@ -123,10 +123,10 @@ template <int PH>
 void launch_m(int lmax, int nb, cudaStream_t st, bool pdl, size_t smem, const StackDesc *desc, const Sched &sc, int stage,
               int j) {
   switch (lmax) {
-    case 2: launch_phase_kernel(k_phase_m<PH, 2>, nb, st, pdl, smem, desc, sc, stage, j); break;
-    case 3: launch_phase_kernel(k_phase_m<PH, 3>, nb, st, pdl, smem, desc, sc, stage, j); break;
-    case 5: launch_phase_kernel(k_phase_m<PH, 5>, nb, st, pdl, smem, desc, sc, stage, j); break;
-    default: launch_phase_kernel(k_phase_m<PH, 8>, nb, st, pdl, smem, desc, sc, stage, j); break;
+    case 2: launch_kernel(k_phase_m<PH, 2>, nb, st, pdl, smem, desc, sc, stage, j); break;
+    case 3: launch_kernel(k_phase_m<PH, 3>, nb, st, pdl, smem, desc, sc, stage, j); break;
+    case 5: launch_kernel(k_phase_m<PH, 5>, nb, st, pdl, smem, desc, sc, stage, j); break;
+    default: launch_kernel(k_phase_m<PH, 8>, nb, st, pdl, smem, desc, sc, stage, j); break;
   }
 }
 

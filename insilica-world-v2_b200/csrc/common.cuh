@@ -179,6 +179,33 @@ struct StageArgs {
   int n;                                     // fast sub-steps of this stage
 };
 
+// Programmatic dependent launch between the kernels of a step: a kernel is launched while the previous one drains, waits
+// for that one's completion and memory before its first read (griddepcontrol.wait; a no-op after a plain launch), and lets
+// its own dependent launch at once (griddepcontrol.launch_dependents).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() {
+  pdl_wait();
+  pdl_trigger();
+}
+
+// Launch a kernel of THREADS-thread blocks, as a programmatic dependent of the kernel before it in the stream if `pdl`
+// (which must then be a kernel that enters with pdl_enter or signals nothing).
+template <class... KA, class... A>
+void launch_kernel(void (*kern)(KA...), int nb, cudaStream_t st, bool pdl, size_t smem, const A &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nb);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  ISW_CUDA(cudaLaunchKernelEx(&cfg, kern, KA(args)...));
+}
+
 inline int blocks_for(long long n, int threads = THREADS) {
   long long b = (n + threads - 1) / threads;
   return (int)(b < 1 ? 1 : b);
