@@ -255,7 +255,7 @@ struct BatchSlot {
 };
 
 struct FastGroup {
-  int begin = 0, count = 0, form = 0;       // its tiles [begin, begin + count) and their precision form
+  int begin = 0, count = 0, form = 0, cap = 0;   // its tiles [begin, begin + count), their form, the kernel's capacity
   size_t smem = 0;
 };
 
@@ -436,17 +436,29 @@ const TileSetDev &tiles_on_device(isw_grid *g, TileCache *c) {
   return t;
 }
 
-// The largest k' <= the probe's k at which every tile fits a block: its cells, edges and own cells' edges the
-// threads' registers, what its threads share `budget` bytes of shared memory (0 if none).
-int fitting_k(const TileSetHost &h, int L, bool mixed, int bps) {
-  const size_t nt = fast_tiles_threads(bps), budget = bps == 2 ? SMEM_TWO : SMEM_ONE;
-  const size_t cm = nt * TILE_C, em = nt * TILE_E, am = nt * TILE_A;
-  for (int kk = h.k; kk >= 1; kk--) {
+// The smallest kernel capacity whose registers hold every tile of a tiling at interval k (-1: none).
+int tiles_cap(const TileSetHost &h, int k, int bps) {
+  const int nt = fast_tiles_threads(bps);
+  for (int cap = 0; cap < 2; cap++) {
     bool ok = true;
     for (int p = 0; p < h.P && ok; p++) {
       const int32_t *nc = &h.ncnt[(size_t)p * (h.k + 1)], *ne = &h.ecnt[(size_t)p * (h.k + 1)];
-      ok = (size_t)nc[kk] <= cm && (size_t)ne[kk] <= em && (size_t)ne[0] <= am &&
-           tile_smem_bytes(nc[kk], ne[kk], nc[1], ne[0], L, mixed) <= budget;
+      ok = nc[k] <= nt * TILE_CAP[cap].C && ne[k] <= nt * TILE_CAP[cap].E && ne[0] <= nt * TILE_CAP[cap].A;
+    }
+    if (ok) return cap;
+  }
+  return -1;
+}
+
+// The largest k' <= the probe's k at which every tile fits a block: its cells, edges and own cells' edges the
+// threads' registers, what its threads share `budget` bytes of shared memory (0 if none).
+int fitting_k(const TileSetHost &h, int L, bool mixed, int bps) {
+  const size_t budget = bps == 2 ? SMEM_TWO : SMEM_ONE;
+  for (int kk = h.k; kk >= 1; kk--) {
+    bool ok = tiles_cap(h, kk, bps) >= 0;
+    for (int p = 0; p < h.P && ok; p++) {
+      const int32_t *nc = &h.ncnt[(size_t)p * (h.k + 1)], *ne = &h.ecnt[(size_t)p * (h.k + 1)];
+      ok = tile_smem_bytes(nc[kk], ne[kk], nc[1], ne[0], L, mixed) <= budget;
     }
     if (ok) return kk;
   }
@@ -627,13 +639,15 @@ bool resident(isw_batch *b, const Tiling &t) {
         smax = std::max(smax, tiles_smem(tiles_for(b->slots[q].layers->grid, t.P[q], t.K[q])->host, b->slots[q].layers->d.L, f == 1));
       }
     if (count.empty()) continue;
-    const void *fn = fast_tiles_kernel(t.bps, f == 1);
-    // the kernel's limit is one setting for every batch: always the most a tile may ask for
-    ISW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(t.bps == 2 ? SMEM_TWO : SMEM_ONE)));
-    int per = 0;
-    ISW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, fast_tiles_threads(t.bps), smax));
-    for (const auto &kv : count)
-      if ((long long)per * b->sms < kv.second) return false;
+    for (int cap = 0; cap < 2; cap++) {
+      const void *fn = fast_tiles_kernel(t.bps, cap, f == 1);
+      // the kernel's limit is one setting for every batch: always the most a tile may ask for
+      ISW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(t.bps == 2 ? SMEM_TWO : SMEM_ONE)));
+      int per = 0;
+      ISW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, fast_tiles_threads(t.bps), smax));
+      for (const auto &kv : count)
+        if ((long long)per * b->sms < kv.second) return false;
+    }
   }
   return true;
 }
@@ -665,7 +679,7 @@ void rebuild(isw_batch *b) {
   const int ngroups = kbest > 0 ? 1 + *std::max_element(best.group.begin(), best.group.end()) : 0;
   std::vector<std::vector<TileRef>> grefs(ngroups);
   std::vector<size_t> gsmem(ngroups, 0);
-  std::vector<int> gform(ngroups, 0);
+  std::vector<int> gform(ngroups, 0), gcap(ngroups, 0);
   std::vector<std::shared_ptr<TileCache>> used_tiles;
   std::vector<std::pair<size_t, int>> gfirst;     // per tiled stack in order: its group, its first tile within the group
   for (auto &sl : b->slots) {
@@ -710,6 +724,7 @@ void rebuild(isw_batch *b) {
       d.tiles = tiles_on_device(sl.layers->grid, tc.get());
       gsmem[g] = std::max(gsmem[g], tiles_smem(tc->host, d.L, form_of(sl) == 1));
       gform[g] = form_of(sl);
+      gcap[g] = std::max(gcap[g], tiles_cap(tc->host, best.K[q], best.bps));
       gfirst.emplace_back((size_t)g, (int)grefs[g].size());
       for (int p = 0; p < best.P[q]; p++) grefs[g].push_back(TileRef{s, p});
     }
@@ -790,6 +805,7 @@ void rebuild(isw_batch *b) {
     fg.count = (int)grefs[g].size();
     fg.smem = gsmem[g];
     fg.form = gform[g];
+    fg.cap = gcap[g];
     refs.insert(refs.end(), grefs[g].begin(), grefs[g].end());
     b->groups.push_back(fg);
   }
@@ -931,7 +947,7 @@ void launch_fast(isw_batch *b, cudaStream_t st, int stage, long long timeout_ns,
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    launch_fast_tiles(b->fast_bps, fg.form == 1, cfg, b->cur, b->d_refs + fg.begin, stage, b->flags, b->status, timeout_ns, fault_block);
+    launch_fast_tiles(b->fast_bps, fg.cap, fg.form == 1, cfg, b->cur, b->d_refs + fg.begin, stage, b->flags, b->status, timeout_ns, fault_block);
     if (fault_block >= 0) break;             // the failure test runs the first group only
   }
 }

@@ -231,10 +231,11 @@ const void *fast_grid_kernel_mixed();
 void launch_fast_grid_mixed(const cudaLaunchConfig_t &cfg, const StackDesc *desc, const Sched &sc, int stage, int nsub,
                             GridBarrier *bar, BatchStatus *status, long long timeout_ns);
 
-// The tiled fast loop (fast_tiles.cu): a form's kernel for `bps` tile blocks per SM, its block size, and its launch.
-const void *fast_tiles_kernel(int bps, bool mixed);
+// The tiled fast loop (fast_tiles.cu): a form's kernel of a capacity for `bps` tile blocks per SM,
+// its block size, and its launch.
+const void *fast_tiles_kernel(int bps, int cap, bool mixed);
 int fast_tiles_threads(int bps);
-void launch_fast_tiles(int bps, bool mixed, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
+void launch_fast_tiles(int bps, int cap, bool mixed, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
                        unsigned *flags, BatchStatus *status, long long timeout_ns, int fault_block);
 
 }  // namespace bt

@@ -77,10 +77,10 @@ __device__ __forceinline__ double slot_flux(const double *fl, unsigned v) {
 }
 __device__ __forceinline__ float slot_flux(const float *fl, unsigned v) { return fl[v]; }
 
-template <int NT>
+template <int NT, int CAP>
 __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, unsigned *flags, BatchStatus *status,
                                           long long timeout_ns, bool skip, unsigned char *smem, const int *cnt) {
-  constexpr int CM = TILE_C, EM = TILE_E, AM = TILE_A;
+  constexpr int CM = TILE_CAP[CAP].C, EM = TILE_CAP[CAP].E, AM = TILE_CAP[CAP].A;
   const LayersDev &M = d.M;
   const TileSetDev &T = d.tiles;
   const int k = T.k, n = d.n[st], t = threadIdx.x;
@@ -344,10 +344,10 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
 
 // The mixed form: deviations deta = eta - eta0 and dub = ub - ub0 from zero in FP32, ub0's divergence c0 formed once per
 // cell, the edges' sums of dub in FP64; the layer fluxes, thicknesses and final winds in FP64.
-template <int NT>
+template <int NT, int CAP>
 __device__ __forceinline__ void tile_mixed(const StackDesc &d, int p, int st, unsigned *flags, BatchStatus *status,
                                            long long timeout_ns, bool skip, unsigned char *smem, const int *cnt) {
-  constexpr int CM = TILE_C, EM = TILE_E, AM = TILE_A;
+  constexpr int CM = TILE_CAP[CAP].C, EM = TILE_CAP[CAP].E, AM = TILE_CAP[CAP].A;
   const LayersDev &M = d.M;
   const TileSetDev &T = d.tiles;
   const int k = T.k, n = d.n[st], t = threadIdx.x;
@@ -634,8 +634,8 @@ __device__ __forceinline__ void tile_mixed(const StackDesc &d, int p, int st, un
   if (st == 2 && !finite) raise_status(status, ISW_ENOTFINITE);
 }
 
-template <int NT, bool MIXED>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_fast_tiles(const StackDesc *__restrict__ S, const TileRef *__restrict__ refs,
+template <int NT, int CAP, bool MIXED>
+__global__ void __launch_bounds__(NT, TILE_NT1 / NT) k_fast_tiles(const StackDesc *__restrict__ S, const TileRef *__restrict__ refs,
                                                               int st, unsigned *flags, BatchStatus *status, long long timeout_ns,
                                                               int fault_block) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -650,26 +650,29 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_fast_tiles(const StackDesc *_
   __syncthreads();
   const bool skip = (int)blockIdx.x == fault_block;
   unsigned *own = flags + (size_t)d.tile_base * FLAG_STRIDE;
-  if (MIXED) tile_mixed<NT>(d, tr.p, st, own, status, timeout_ns, skip, smem, cnt);
-  else tile_fp64<NT>(d, tr.p, st, own, status, timeout_ns, skip, smem, cnt);
+  if (MIXED) tile_mixed<NT, CAP>(d, tr.p, st, own, status, timeout_ns, skip, smem, cnt);
+  else tile_fp64<NT, CAP>(d, tr.p, st, own, status, timeout_ns, skip, smem, cnt);
 }
 
 using Kernel = void (*)(const StackDesc *, const TileRef *, int, unsigned *, BatchStatus *, long long, int);
 
+template <int CAP>
 Kernel kernel_for(int bps, bool mixed) {
-  if (bps == 2) return mixed ? k_fast_tiles<TILE_NT2, true> : k_fast_tiles<TILE_NT2, false>;
-  return mixed ? k_fast_tiles<TILE_NT1, true> : k_fast_tiles<TILE_NT1, false>;
+  if (bps == 2) return mixed ? k_fast_tiles<TILE_NT2, CAP, true> : k_fast_tiles<TILE_NT2, CAP, false>;
+  return mixed ? k_fast_tiles<TILE_NT1, CAP, true> : k_fast_tiles<TILE_NT1, CAP, false>;
 }
+
+Kernel kernel_for(int bps, int cap, bool mixed) { return cap == 0 ? kernel_for<0>(bps, mixed) : kernel_for<1>(bps, mixed); }
 
 }  // namespace
 
-const void *fast_tiles_kernel(int bps, bool mixed) { return (const void *)kernel_for(bps, mixed); }
+const void *fast_tiles_kernel(int bps, int cap, bool mixed) { return (const void *)kernel_for(bps, cap, mixed); }
 
 int fast_tiles_threads(int bps) { return bps == 2 ? TILE_NT2 : TILE_NT1; }
 
-void launch_fast_tiles(int bps, bool mixed, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
+void launch_fast_tiles(int bps, int cap, bool mixed, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
                        unsigned *flags, BatchStatus *status, long long timeout_ns, int fault_block) {
-  ISW_CUDA(cudaLaunchKernelEx(&cfg, kernel_for(bps, mixed), desc, refs, stage, flags, status, timeout_ns, fault_block));
+  ISW_CUDA(cudaLaunchKernelEx(&cfg, kernel_for(bps, cap, mixed), desc, refs, stage, flags, status, timeout_ns, fault_block));
 }
 
 }  // namespace bt

@@ -19,11 +19,15 @@
 namespace isw {
 
 // What one tile may hold: thread t of a block of NT keeps the state of cells t, t + NT, ... and edges t, t + NT, ... in
-// registers (64 a thread), so a tile has at most TILE_C x NT cells, TILE_E x NT edges and TILE_A x NT edges of its own
-// cells, whose sub-step sums are kept. Five edges a thread let a level-7 stack (163,842 cells) fill 148 SMs.
-constexpr int TILE_C = 2, TILE_E = 5, TILE_A = 4;
+// registers (80 a thread), so a tile has at most C x NT cells, E x NT edges and A x NT edges of its own cells, whose
+// sub-step sums are kept. Two capacities, a kernel each: the small one keeps all of it in registers, the large one (which
+// lets a level-7 stack of 163,842 cells fill 148 SMs) spills some.
+struct TileCap {
+  int C, E, A;
+};
+constexpr TileCap TILE_CAP[2] = {{2, 5, 3}, {2, 7, 5}};
 // Threads of a tile block when one or two tiles share an SM.
-constexpr int TILE_NT1 = 1024, TILE_NT2 = 512;
+constexpr int TILE_NT1 = 768, TILE_NT2 = 384;
 constexpr int TILE_FLAG_STRIDE = 8;            // a tile's exchange flag has a 32-byte sector of its own
 
 struct TileSetHost {
