@@ -151,21 +151,25 @@ __global__ void __launch_bounds__(THREADS) k_phase(const StackDesc *__restrict__
     if (EXT && M.air && d.theta && (M.vmix != 0 || M.vmix_cd != 0) && d.L > 1)
       ISW_BATCH_L(d.L, LMAXK, fp64::vmix_heat_cell<LL>(M, d.h, d.theta, i));
   } else if (PH == PH_HF1) {
-    ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 1, i / M.g.E, i % M.g.E));
+    const EdgeRow r = edge_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
   } else if (PH == PH_POST) {
     if (kind == 1) {
       if ((M.vmix != 0 || M.vmix_cd != 0) && d.L > 1) ISW_BATCH_L(d.L, LMAXK, fp64::vmix_edge<LL, EXT>(M, d.h, d.u, d.dt, i));
     } else {
-      ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 1, i / M.g.E, i % M.g.E));
+      const EdgeRow r = edge_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
     }
   } else if (PH == PH_P1) {
     ISW_BATCH_L(d.L, LMAXK, fp64::tr_c1<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
   } else if (PH == PH_P2E) {
-    ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 2, i / M.g.E, i % M.g.E));
+    const EdgeRow r = edge_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 2, r.j0, r.j1, r.e));
   } else if (PH == PH_P2) {
     ISW_BATCH_L(d.L, LMAXK, fp64::tr_c2<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
   } else if (PH == PH_P3E) {
-    ISW_BATCH_L(d.L, LMAXK, fp64::tr_a_edge<LL>(d.T, d.tr, i / M.g.E, i % M.g.E));
+    const EdgeRow r = edge_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, fp64::tr_a_edge<LL>(d.T, d.tr, r.j0, r.j1, r.e));
   } else if (PH == PH_P3) {
     ISW_BATCH_L(d.L, LMAXK, fp64::tr_c3<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
   } else if (PH == PH_P4) {
@@ -661,6 +665,9 @@ void rebuild(isw_batch *b) {
   int untiled[2] = {0, 0};
   size_t s_smem[2] = {0, 0};
   const double cs[3] = {1.0 / 3.0, 1.0 / 2.0, 1.0};
+  long long edge_items[2] = {0, 0};                                     // per form: (tracer, edge) pairs
+  for (auto &sl : b->slots)
+    if (sl.used && sl.tr) edge_items[form_of(sl)] += (long long)sl.ntr * sl.layers->grid->d.E;
   int used = 0;
   for (auto &sl : b->slots) used += sl.used ? 1 : 0;
   Tiling best;
@@ -750,7 +757,10 @@ void rebuild(isw_batch *b) {
       chunks(uedge[f], d.M.g.E);
     }
     if (d.has_tr) chunks(rows[f], sl.ntr * d.M.g.N);       // (tracer, cell) pairs
-    if (d.has_tr) chunks(erows[f], sl.ntr * d.M.g.E);      // (tracer, edge) pairs
+    if (d.has_tr) {                                        // (tracers of a thread, edge)
+      d.eg = fp64::tracers_a_thread(edge_items[f], sl.ntr);
+      chunks(erows[f], (sl.ntr + d.eg - 1) / d.eg * d.M.g.E);
+    }
     desc.push_back(d);
   }
   b->nstacks = (int)desc.size();

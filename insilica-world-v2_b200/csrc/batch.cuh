@@ -31,6 +31,7 @@ struct StackDesc {
   double *theta;             // air layers: potential temperature (L x N); null for Boussinesq layers
   double dt;
   int L, has_tr, tiled;
+  int eg;                    // tracers of one thread of the transport's edge passes
   int s_stage;               // the slow tendency stages its blocks' neighbour records in shared memory
   int n[3];
   double cdt[3], tau[3], inv_n[3];
@@ -174,6 +175,15 @@ __device__ __forceinline__ const StackDesc &stage_desc(const StackDesc *S, int s
 // last sub-step); PH_CS and PH_D: their limiter and their stage's end (tiled stacks end their stage in the tile kernel).
 enum Phase { PH_INIT, PH_LAPE1, PH_LAPCV, PH_LAPE2, PH_A, PH_E, PH_S, PH_ETA, PH_UF, PH_CS, PH_D, PH_POST, PH_P2, PH_P3, PH_P4,
              PH_P1, PH_P2E, PH_P3E, PH_VMIX, PH_HF1, PH_VHEAT, PH_ONBED };
+
+// Item i of the transport's edge passes: its edge, and its tracers [j0, j1).
+struct EdgeRow {
+  int j0, j1, e;
+};
+__device__ __forceinline__ EdgeRow edge_row(const StackDesc &d, int i) {
+  const int g = i / d.M.g.E, ntr = d.tr.rows / d.L, j0 = g * d.eg;
+  return EdgeRow{j0, min(j0 + d.eg, ntr), i - g * d.M.g.E};
+}
 
 // Domains of a phase, in block order: which chunk tables its blocks walk.
 template <int PH>

@@ -94,21 +94,25 @@ __global__ void __launch_bounds__(THREADS) k_phase_m(const StackDesc *__restrict
   } else if (PH == PH_VMIX) {
     if ((M.vmix != 0 || M.vmix_cd != 0) && d.L > 1) ISW_BATCH_L(d.L, LMAXK, fp64::vmix_edge<LL, false>(M, d.h, d.u, d.dt, i));
   } else if (PH == PH_HF1) {
-    ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 1, i / M.g.E, i % M.g.E));
+    const EdgeRow r = edge_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
   } else if (PH == PH_POST) {
     if (kind == 1) {
       if ((M.vmix != 0 || M.vmix_cd != 0) && d.L > 1) ISW_BATCH_L(d.L, LMAXK, fp64::vmix_edge<LL, false>(M, d.h, d.u, d.dt, i));
     } else {
-      ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 1, i / M.g.E, i % M.g.E));
+      const EdgeRow r = edge_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
     }
   } else if (PH == PH_P1) {
     ISW_BATCH_L(d.L, LMAXK, mixed::tr_c1<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
   } else if (PH == PH_P2E) {
-    ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 2, i / M.g.E, i % M.g.E));
+    const EdgeRow r = edge_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 2, r.j0, r.j1, r.e));
   } else if (PH == PH_P2) {
     ISW_BATCH_L(d.L, LMAXK, mixed::tr_c2<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
   } else if (PH == PH_P3E) {
-    ISW_BATCH_L(d.L, LMAXK, mixed::tr_a_edge<LL>(d.T, d.tr, i / M.g.E, i % M.g.E));
+    const EdgeRow r = edge_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, mixed::tr_a_edge<LL>(d.T, d.tr, r.j0, r.j1, r.e));
   } else if (PH == PH_P3) {
     ISW_BATCH_L(d.L, LMAXK, mixed::tr_c3<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
   } else if (PH == PH_P4) {

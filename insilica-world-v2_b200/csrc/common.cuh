@@ -44,6 +44,9 @@ struct GridDev {
   int N, E, NV, nE2;              // nE2 = eoeStart[E], the length of the TRiSK CSR
   const int *eI, *eJ, *nbr, *cellEdge, *cellEdgeAsc, *ev1, *ev2, *vEdge, *vCell, *eoeStart, *eoe, *d2idx;
   const int2 *eIJ;                // (eI, eJ) per edge, one 8-byte load
+  // per cell, in ascending edge order (6 slots, pads -1): 2 x edge + (1 where the cell is the edge's eJ side), and the cell
+  // on the edge's other side; what cellEdgeAsc with eI and eJ of every edge would say, in a quarter of the loads
+  const int *ascE, *ascN;
   const int8_t *cellSign, *vEdgeSign, *vSlot;
   const double *le, *de, *areaCell, *areaV, *fV, *kite, *w, *d2wt;
   const float *w32, *d2wt32, *le32, *de32, *rde32, *rle32, *rA32, *rAV32, *kite32;

@@ -172,6 +172,19 @@ static isw_grid *grid_create(const isw_grid_host *h, int device) {
       for (int e = 0; e < E; e++) { eij[2 * (size_t)e] = h->eI[e]; eij[2 * (size_t)e + 1] = h->eJ[e]; }
       d.eIJ = reinterpret_cast<const int2 *>(upload(g, eij.data(), eij.size()));
     }
+    {
+      std::vector<int32_t> ae((size_t)N * 6, -1), an((size_t)N * 6, -1);
+      for (int i = 0; i < N; i++)
+        for (int q = 0; q < 6; q++) {
+          const int e = h->cellEdgeAsc[(size_t)i * 6 + q];
+          if (e < 0) continue;
+          const bool in = h->eI[e] != i;
+          ae[(size_t)i * 6 + q] = 2 * e + (in ? 1 : 0);
+          an[(size_t)i * 6 + q] = in ? h->eI[e] : h->eJ[e];
+        }
+      d.ascE = upload(g, ae.data(), ae.size());
+      d.ascN = upload(g, an.data(), an.size());
+    }
     d.nbr = upload(g, h->nbr, (size_t)N * 6);
     d.cellEdge = upload(g, h->cellEdge, (size_t)N * 6);
     d.cellEdgeAsc = upload(g, h->cellEdgeAsc, (size_t)N * 6);

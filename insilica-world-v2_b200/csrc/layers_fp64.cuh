@@ -591,12 +591,12 @@ __device__ __forceinline__ void scale_sum_cell(const LayersDev &M, const StageAr
 #pragma unroll
   for (int k = 0; k < L; k++) out[k] = 0;
   int es[6];
-  slots6(g.cellEdgeAsc, i, es);
+  slots6(g.ascE, i, es);
 #pragma unroll
   for (int s = 0; s < 6; s++) {
-    const int e = es[s];
-    if (e < 0) continue;
-    const bool mine = g.eI[e] == i;
+    if (es[s] < 0) continue;
+    const int e = es[s] >> 1;
+    const bool mine = (es[s] & 1) == 0;
     const double le = g.le[e];
 #pragma unroll
     for (int k = 0; k < L; k++) {

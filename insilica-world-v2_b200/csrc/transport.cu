@@ -50,18 +50,19 @@ __global__ void __launch_bounds__(THREADS) k_p1(const TransportDev T, const TrAr
   ISW_TR_L(a.L, fp64::tr_p1<LL>(T, a, order, false, t / T.g.N, t % T.g.N));
 }
 
-__global__ void __launch_bounds__(THREADS) k_hf(const TransportDev T, const TrArgs a, int ntr, int stage) {
+// one thread per (eg tracers, edge)
+__global__ void __launch_bounds__(THREADS) k_hf(const TransportDev T, const TrArgs a, int ntr, int eg, int stage) {
   pdl_enter();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.g.E * ntr) return;
-  ISW_TR_L(a.L, fp64::tr_hf_edge<LL>(T, a, stage, t / T.g.E, t % T.g.E));
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j0 = t / T.g.E * eg;
+  if (j0 >= ntr) return;
+  ISW_TR_L(a.L, fp64::tr_hf_edge<LL>(T, a, stage, j0, min(j0 + eg, ntr), t % T.g.E));
 }
 
-__global__ void __launch_bounds__(THREADS) k_aflux(const TransportDev T, const TrArgs a, int ntr) {
+__global__ void __launch_bounds__(THREADS) k_aflux(const TransportDev T, const TrArgs a, int ntr, int eg) {
   pdl_enter();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.g.E * ntr) return;
-  ISW_TR_L(a.L, fp64::tr_a_edge<LL>(T, a, t / T.g.E, t % T.g.E));
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j0 = t / T.g.E * eg;
+  if (j0 >= ntr) return;
+  ISW_TR_L(a.L, fp64::tr_a_edge<LL>(T, a, j0, min(j0 + eg, ntr), t % T.g.E));
 }
 
 __global__ void __launch_bounds__(THREADS) k_c1(const TransportDev T, const TrArgs a, int ntr) {
@@ -200,18 +201,19 @@ int isw_transport_step_many(isw_transport *t, const double *M0, const double *M1
       a.tr[j] = tracers[j];
     }
     cudaStream_t st = (cudaStream_t)stream;
-    const int nb = blocks_for((long long)t->d.g.N * ntr), ne = blocks_for((long long)t->d.g.E * ntr);
+    const int eg = fp64::tracers_a_thread((long long)t->d.g.E * ntr, ntr);
+    const int nb = blocks_for((long long)t->d.g.N * ntr), ne = blocks_for((long long)t->d.g.E * ((ntr + eg - 1) / eg));
     // the first kernel takes plain stream order, the others are programmatic dependents of the one before (8 tracers of 5
     // layers at level 6: 345 -> 334 us)
     if (order == 1) {
       launch_kernel(k_p1, nb, st, false, 0, t->d, a, ntr, order);
       launch_kernel(k_td_out, blocks_for((long long)t->d.g.N * a.rows), st, true, 0, t->d, a);
     } else {
-      launch_kernel(k_hf, ne, st, false, 0, t->d, a, ntr, 1);
+      launch_kernel(k_hf, ne, st, false, 0, t->d, a, ntr, eg, 1);
       launch_kernel(k_c1, nb, st, true, 0, t->d, a, ntr);
-      launch_kernel(k_hf, ne, st, true, 0, t->d, a, ntr, 2);
+      launch_kernel(k_hf, ne, st, true, 0, t->d, a, ntr, eg, 2);
       launch_kernel(k_c2, nb, st, true, 0, t->d, a, ntr);
-      launch_kernel(k_aflux, ne, st, true, 0, t->d, a, ntr);
+      launch_kernel(k_aflux, ne, st, true, 0, t->d, a, ntr, eg);
       launch_kernel(k_c3, nb, st, true, 0, t->d, a, ntr);
       launch_kernel(k_p4, nb, st, true, 0, t->d, a, ntr);
     }

@@ -177,29 +177,36 @@ __device__ __forceinline__ void load_stencil_layers(const F *__restrict__ fld, i
   }
 }
 
-// A cell's edges in ascending edge order (cellEdgeAsc), with their two cells.
+// A cell's edges in ascending edge order: the edge (-1: a padded slot), whether it leaves the cell (the cell is its eI
+// side), the cell on its other side.
 struct CellEdges {
-  int e[6], a[6], b[6];
+  int e[6], nb[6];
+  bool out[6];
 };
 
+template <bool NB = true>
 __device__ __forceinline__ void load_edges(const GridDev &g, int i, CellEdges &c) {
-  slots6(g.cellEdgeAsc, i, c.e);
+  int v[6];
+  slots6(g.ascE, i, v);
+  if (NB) slots6(g.ascN, i, c.nb);
 #pragma unroll
   for (int s = 0; s < 6; s++) {
-    const int e = c.e[s];
-    c.a[s] = e >= 0 ? g.eI[e] : 0;
-    c.b[s] = e >= 0 ? g.eJ[e] : 0;
+    c.e[s] = v[s] >> 1;
+    c.out[s] = (v[s] & 1) == 0;
   }
 }
 
 // reference trisk.cu:48-59
 __device__ __forceinline__ double mass_cell(const GridDev &g, const double *__restrict__ M0, const double *__restrict__ Fml, int l, int i) {
   double m = M0[(size_t)l * g.N + i];
-  for (int k = 0; k < 6; k++) {
-    const int e = g.cellEdgeAsc[i * 6 + k];
-    if (e < 0) break;
-    if (g.eI[e] == i) m -= Fml[e]; else m += Fml[e];
-  }
+  CellEdges c;
+  load_edges<false>(g, i, c);
+#pragma unroll
+  for (int q = 0; q < 6; q++)
+    if (c.e[q] >= 0) {
+      const double f = Fml[c.e[q]];
+      if (c.out[q]) m -= f; else m += f;
+    }
   return m;
 }
 
@@ -211,11 +218,12 @@ __device__ __forceinline__ void tr_p1(const TransportDev &T, const TrArgs &a, in
   const int N = g.N, E = g.E;
   CellEdges c;
   load_edges(g, i, c);
-  double m1[L], td[L], s[L], mx[L];
+  double m1[L], td[L], s[L], mx[L], own[L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
     const double m0 = a.M0[om], pi = a.tr[j][om];
+    own[l] = pi;
     m1[l] = m0;
     td[l] = m0 * pi;
     s[l] = m0 * pi;
@@ -226,7 +234,7 @@ __device__ __forceinline__ void tr_p1(const TransportDev &T, const TrArgs &a, in
   for (int q = 0; q < 6; q++) {
     const int e = c.e[q];
     if (e >= 0) {
-      const bool out = c.a[q] == i;
+      const bool out = c.out[q];
       Stencil stn;
       if (order != 1) load_stencil(g, e, stn);
 #pragma unroll
@@ -234,7 +242,8 @@ __device__ __forceinline__ void tr_p1(const TransportDev &T, const TrArgs &a, in
         const double *p = a.tr[j] + (size_t)l * N;
         const double f = a.Fm[(size_t)l * E + e];
         if (with_mass) { if (out) m1[l] -= f; else m1[l] += f; }
-        const double pa = p[c.a[q]], pb = p[c.b[q]];
+        const double pn = p[c.nb[q]];
+        const double pa = out ? own[l] : pn, pb = out ? pn : own[l];
         const double fu = upwind_v(f, pa, pb);
         if (out) td[l] -= fu; else td[l] += fu;
         if (order != 1) {
@@ -279,8 +288,8 @@ __device__ __forceinline__ void tr_p4(const TransportDev &T, const TrArgs &a, in
   for (int q = 0; q < 6; q++) {
     const int e = c.e[q];
     if (e >= 0) {
-      const bool out = c.a[q] == i;
-      const int nb = out ? c.b[q] : c.a[q];
+      const bool out = c.out[q];
+      const int nb = c.nb[q];
       double Av[L], rpn[L], rmn[L];
       ld_layers<L>(T.A + fx(j, E, e, L), Av);
       ld_layers<L>(T.Rp + fx(j, N, nb, L), rpn);
@@ -305,49 +314,67 @@ __device__ __forceinline__ void tr_p4(const TransportDev &T, const TrArgs &a, in
 // stage-1 fluxes, then the stage-2 fluxes, then the antidiffusive fluxes. The tracers are read in place until the
 // limited update overwrites them, so no copy of them is kept. ----
 
-// stage = 1: fluxes of the tracer itself; 2: of p1. A[j][e][l] = hoflux(f, field) for every layer.
+// Tracers of one thread of the edge passes: every tracer of an edge reads the same stencil row and fluxes (104 + 8 L bytes
+// and 11 of some 30 loads), so a thread takes as many as still leave EDGE_THREADS threads (768 on each of 148 SMs).
+constexpr long long EDGE_THREADS = 148 * 768;
+__host__ __device__ inline int tracers_a_thread(long long items, int ntr) {
+  const long long g = items / EDGE_THREADS;
+  return g < 1 ? 1 : g < ntr ? (int)g : ntr;
+}
+
+// stage = 1: fluxes of the tracer itself; 2: of p1. A[j][e][l] = hoflux(f, field) for every layer of tracers j0 .. j1 - 1.
 template <int L>
-__device__ __forceinline__ void tr_hf_edge(const TransportDev &T, const TrArgs &a, int stage, int j, int e) {
+__device__ __forceinline__ void tr_hf_edge(const TransportDev &T, const TrArgs &a, int stage, int j0, int j1, int e) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
-  const int ea = g.eI[e], eb = g.eJ[e];
+  const int2 ab = g.eIJ[e];
   Stencil stn;
   load_stencil(g, e, stn);
-  double out[L];
-  if (stage == 1) {
+  double f[L];
+#pragma unroll
+  for (int l = 0; l < L; l++) f[l] = a.Fm[(size_t)l * E + e];
+#pragma unroll 1
+  for (int j = j0; j < j1; j++) {
+    double out[L];
+    if (stage == 1) {
+#pragma unroll
+      for (int l = 0; l < L; l++) {
+        const double *p = a.tr[j] + (size_t)l * N;
+        out[l] = hoflux_s(f[l], p, stn, p[ab.x], p[ab.y], a.beta);
+      }
+    } else {
+      StencilLayers<L, double> v;
+      load_stencil_layers<L>(T.p1, j, N, ab.x, ab.y, stn.o, v);
+#pragma unroll
+      for (int l = 0; l < L; l++) out[l] = hoflux_v(f[l], stn, v.pa[l], v.pb[l], v.q0[l], v.q1[l], v.q2[l], v.q3[l], a.beta);
+    }
+    st_layers<L>(T.A + fx(j, E, e, L), out);
+  }
+}
+
+// the antidiffusive flux A = hoflux(p2) - upwind(psi) of every layer of edge e, tracers j0 .. j1 - 1
+template <int L>
+__device__ __forceinline__ void tr_a_edge(const TransportDev &T, const TrArgs &a, int j0, int j1, int e) {
+  const GridDev &g = T.g;
+  const int N = g.N, E = g.E;
+  const int2 ab = g.eIJ[e];
+  Stencil stn;
+  load_stencil(g, e, stn);
+  double f[L];
+#pragma unroll
+  for (int l = 0; l < L; l++) f[l] = a.Fm[(size_t)l * E + e];
+#pragma unroll 1
+  for (int j = j0; j < j1; j++) {
+    StencilLayers<L, double> v;
+    load_stencil_layers<L>(T.p2, j, N, ab.x, ab.y, stn.o, v);
+    double out[L];
 #pragma unroll
     for (int l = 0; l < L; l++) {
       const double *p = a.tr[j] + (size_t)l * N;
-      out[l] = hoflux_s(a.Fm[(size_t)l * E + e], p, stn, p[ea], p[eb], a.beta);
+      out[l] = hoflux_v(f[l], stn, v.pa[l], v.pb[l], v.q0[l], v.q1[l], v.q2[l], v.q3[l], a.beta) - upwind_v(f[l], p[ab.x], p[ab.y]);
     }
-  } else {
-    StencilLayers<L, double> v;
-    load_stencil_layers<L>(T.p1, j, N, ea, eb, stn.o, v);
-#pragma unroll
-    for (int l = 0; l < L; l++)
-      out[l] = hoflux_v(a.Fm[(size_t)l * E + e], stn, v.pa[l], v.pb[l], v.q0[l], v.q1[l], v.q2[l], v.q3[l], a.beta);
+    st_layers<L>(T.A + fx(j, E, e, L), out);
   }
-  st_layers<L>(T.A + fx(j, E, e, L), out);
-}
-
-// the antidiffusive flux A = hoflux(p2) - upwind(psi) of every layer of (tracer j, edge e)
-template <int L>
-__device__ __forceinline__ void tr_a_edge(const TransportDev &T, const TrArgs &a, int j, int e) {
-  const GridDev &g = T.g;
-  const int N = g.N, E = g.E;
-  const int ea = g.eI[e], eb = g.eJ[e];
-  Stencil stn;
-  load_stencil(g, e, stn);
-  StencilLayers<L, double> v;
-  load_stencil_layers<L>(T.p2, j, N, ea, eb, stn.o, v);
-  double out[L];
-#pragma unroll
-  for (int l = 0; l < L; l++) {
-    const double *p = a.tr[j] + (size_t)l * N;
-    const double f = a.Fm[(size_t)l * E + e];
-    out[l] = hoflux_v(f, stn, v.pa[l], v.pb[l], v.q0[l], v.q1[l], v.q2[l], v.q3[l], a.beta) - upwind_v(f, p[ea], p[eb]);
-  }
-  st_layers<L>(T.A + fx(j, E, e, L), out);
 }
 
 // cell pass of stage 1: td and p1 from the stage-1 edge fluxes; with_mass: M1 formed here (tracer 0 stores it), else
@@ -358,11 +385,12 @@ __device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, in
   const int N = g.N, E = g.E;
   CellEdges c;
   load_edges(g, i, c);
-  double m1[L], td[L], s[L], mx[L];
+  double m1[L], td[L], s[L], mx[L], own[L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
     const double m0 = a.M0[om], pi = a.tr[j][om];
+    own[l] = pi;
     m1[l] = m0;
     td[l] = m0 * pi;
     s[l] = m0 * pi;
@@ -373,14 +401,15 @@ __device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, in
   for (int q = 0; q < 6; q++) {
     const int e = c.e[q];
     if (e >= 0) {
-      const bool out = c.a[q] == i;
+      const bool out = c.out[q];
       double Av[L];
       ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll
       for (int l = 0; l < L; l++) {
         const double *p = a.tr[j] + (size_t)l * N;
         const double f = a.Fm[(size_t)l * E + e];
-        const double fu = upwind_v(f, p[c.a[q]], p[c.b[q]]);
+        const double pn = p[c.nb[q]];
+        const double fu = upwind_v(f, out ? own[l] : pn, out ? pn : own[l]);
         const double hf = frac * Av[l];
         const double m = frac * f;
         if (out) { m1[l] -= f; td[l] -= fu; s[l] -= hf; mx[l] -= m; }
@@ -408,7 +437,7 @@ __device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, in
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
   CellEdges c;
-  load_edges(g, i, c);
+  load_edges<false>(g, i, c);
   double s[L], mx[L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
@@ -421,7 +450,7 @@ __device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, in
   for (int q = 0; q < 6; q++) {
     const int e = c.e[q];
     if (e >= 0) {
-      const bool out = c.a[q] == i;
+      const bool out = c.out[q];
       double Av[L];
       ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll
@@ -444,8 +473,9 @@ template <int L>
 __device__ __forceinline__ void tr_c3(const TransportDev &T, const TrArgs &a, int j, int i) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
-  int es[6], nb[6];
-  slots6(g.cellEdgeAsc, i, es);
+  CellEdges c;
+  load_edges<false>(g, i, c);
+  int nb[6];
   slots6(g.nbr, i, nb);
   double Pp[L], Pm[L], hi[L], lo[L], ti[L];
   ld_layers<L>(T.td + fx(j, N, i, L), ti);
@@ -459,9 +489,9 @@ __device__ __forceinline__ void tr_c3(const TransportDev &T, const TrArgs &a, in
   }
 #pragma unroll
   for (int q = 0; q < 6; q++) {
-    const int e = es[q];
+    const int e = c.e[q];
     if (e >= 0) {
-      const bool out = g.eI[e] == i;
+      const bool out = c.out[q];
       double Av[L];
       ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll

@@ -75,8 +75,8 @@ __device__ __forceinline__ void tr_p4(const TransportDev &T, const TrArgs &a, in
   for (int q = 0; q < 6; q++) {
     const int e = c.e[q];
     if (e >= 0) {
-      const bool out = c.a[q] == i;
-      const int nb = out ? c.b[q] : c.a[q];
+      const bool out = c.out[q];
+      const int nb = c.nb[q];
       float Av[L], rpn[L], rmn[L];
       ld_layers<L>(T.Af + fx(j, E, e, L), Av);
       ld_layers<L>(T.Rpf + fx(j, N, nb, L), rpn);
@@ -101,49 +101,59 @@ __device__ __forceinline__ void tr_p4(const TransportDev &T, const TrArgs &a, in
 // fluxes of the edge passes are stored in FP64 (T.A), the antidiffusive fluxes rounded to FP32 once (T.Af). ----
 
 template <int L>
-__device__ __forceinline__ void tr_hf_edge(const TransportDev &T, const TrArgs &a, int stage, int j, int e) {
+__device__ __forceinline__ void tr_hf_edge(const TransportDev &T, const TrArgs &a, int stage, int j0, int j1, int e) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
-  const int ea = g.eI[e], eb = g.eJ[e];
+  const int2 ab = g.eIJ[e];
   const float beta = (float)a.beta;
   Stencil32 stn;
   load_stencil(g, e, stn);
-  double out[L];
-  if (stage == 1) {
+  double f[L];
 #pragma unroll
-    for (int l = 0; l < L; l++) {
-      const double *p = a.tr[j] + (size_t)l * N;
-      out[l] = hoflux(a.Fm[(size_t)l * E + e], p, stn, p[ea], p[eb], beta);
+  for (int l = 0; l < L; l++) f[l] = a.Fm[(size_t)l * E + e];
+#pragma unroll 1
+  for (int j = j0; j < j1; j++) {
+    double out[L];
+    if (stage == 1) {
+#pragma unroll
+      for (int l = 0; l < L; l++) {
+        const double *p = a.tr[j] + (size_t)l * N;
+        out[l] = hoflux(f[l], p, stn, p[ab.x], p[ab.y], beta);
+      }
+    } else {
+      fp64::StencilLayers<L, float> v;
+      fp64::load_stencil_layers<L>(T.p1f, j, N, ab.x, ab.y, stn.o, v);
+#pragma unroll
+      for (int l = 0; l < L; l++) out[l] = hoflux_v(f[l], stn, v.pa[l], v.pb[l], v.q0[l], v.q1[l], v.q2[l], v.q3[l], beta);
     }
-  } else {
-    fp64::StencilLayers<L, float> v;
-    fp64::load_stencil_layers<L>(T.p1f, j, N, ea, eb, stn.o, v);
-#pragma unroll
-    for (int l = 0; l < L; l++)
-      out[l] = hoflux_v(a.Fm[(size_t)l * E + e], stn, v.pa[l], v.pb[l], v.q0[l], v.q1[l], v.q2[l], v.q3[l], beta);
+    st_layers<L>(T.A + fx(j, E, e, L), out);
   }
-  st_layers<L>(T.A + fx(j, E, e, L), out);
 }
 
 template <int L>
-__device__ __forceinline__ void tr_a_edge(const TransportDev &T, const TrArgs &a, int j, int e) {
+__device__ __forceinline__ void tr_a_edge(const TransportDev &T, const TrArgs &a, int j0, int j1, int e) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
-  const int ea = g.eI[e], eb = g.eJ[e];
+  const int2 ab = g.eIJ[e];
   const float beta = (float)a.beta;
   Stencil32 stn;
   load_stencil(g, e, stn);
-  fp64::StencilLayers<L, float> v;
-  fp64::load_stencil_layers<L>(T.p2f, j, N, ea, eb, stn.o, v);
-  float out[L];
+  double f[L];
 #pragma unroll
-  for (int l = 0; l < L; l++) {
-    const double *p = a.tr[j] + (size_t)l * N;
-    const double f = a.Fm[(size_t)l * E + e];
-    out[l] = (float)(hoflux_v(f, stn, v.pa[l], v.pb[l], v.q0[l], v.q1[l], v.q2[l], v.q3[l], beta) -
-                     fp64::upwind_v(f, p[ea], p[eb]));
+  for (int l = 0; l < L; l++) f[l] = a.Fm[(size_t)l * E + e];
+#pragma unroll 1
+  for (int j = j0; j < j1; j++) {
+    fp64::StencilLayers<L, float> v;
+    fp64::load_stencil_layers<L>(T.p2f, j, N, ab.x, ab.y, stn.o, v);
+    float out[L];
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+      const double *p = a.tr[j] + (size_t)l * N;
+      out[l] = (float)(hoflux_v(f[l], stn, v.pa[l], v.pb[l], v.q0[l], v.q1[l], v.q2[l], v.q3[l], beta) -
+                       fp64::upwind_v(f[l], p[ab.x], p[ab.y]));
+    }
+    st_layers<L>(T.Af + fx(j, E, e, L), out);
   }
-  st_layers<L>(T.Af + fx(j, E, e, L), out);
 }
 
 template <int L>
@@ -152,11 +162,12 @@ __device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, in
   const int N = g.N, E = g.E;
   fp64::CellEdges c;
   fp64::load_edges(g, i, c);
-  double m1[L], td[L], s[L], mx[L];
+  double m1[L], td[L], s[L], mx[L], own[L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
     const double m0 = a.M0[om], pi = a.tr[j][om];
+    own[l] = pi;
     m1[l] = m0;
     td[l] = m0 * pi;
     s[l] = m0 * pi;
@@ -167,14 +178,15 @@ __device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, in
   for (int q = 0; q < 6; q++) {
     const int e = c.e[q];
     if (e >= 0) {
-      const bool out = c.a[q] == i;
+      const bool out = c.out[q];
       double Av[L];
       ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll
       for (int l = 0; l < L; l++) {
         const double *p = a.tr[j] + (size_t)l * N;
         const double f = a.Fm[(size_t)l * E + e];
-        const double fu = fp64::upwind_v(f, p[c.a[q]], p[c.b[q]]);
+        const double pn = p[c.nb[q]];
+        const double fu = fp64::upwind_v(f, out ? own[l] : pn, out ? pn : own[l]);
         const double hf = frac * Av[l];
         const double m = frac * f;
         if (out) { m1[l] -= f; td[l] -= fu; s[l] -= hf; mx[l] -= m; }
@@ -200,7 +212,7 @@ __device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, in
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
   fp64::CellEdges c;
-  fp64::load_edges(g, i, c);
+  fp64::load_edges<false>(g, i, c);
   double s[L], mx[L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
@@ -213,7 +225,7 @@ __device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, in
   for (int q = 0; q < 6; q++) {
     const int e = c.e[q];
     if (e >= 0) {
-      const bool out = c.a[q] == i;
+      const bool out = c.out[q];
       double Av[L];
       ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll
@@ -235,8 +247,9 @@ template <int L>
 __device__ __forceinline__ void tr_c3(const TransportDev &T, const TrArgs &a, int j, int i) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
-  int es[6], nb[6];
-  slots6(g.cellEdgeAsc, i, es);
+  fp64::CellEdges c;
+  fp64::load_edges<false>(g, i, c);
+  int nb[6];
   slots6(g.nbr, i, nb);
   double Pp[L], Pm[L], hi[L], lo[L], ti[L];
   ld_layers<L>(T.td + fx(j, N, i, L), ti);
@@ -250,9 +263,9 @@ __device__ __forceinline__ void tr_c3(const TransportDev &T, const TrArgs &a, in
   }
 #pragma unroll
   for (int q = 0; q < 6; q++) {
-    const int e = es[q];
+    const int e = c.e[q];
     if (e >= 0) {
-      const bool out = g.eI[e] == i;
+      const bool out = c.out[q];
       float Av[L];
       ld_layers<L>(T.Af + fx(j, E, e, L), Av);
 #pragma unroll
