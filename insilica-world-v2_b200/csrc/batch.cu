@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(THREADS) k_phase(const StackDesc *__restrict__
     const StageArgs a = stage_args(d, st);
     if (kind == 0) {
       ISW_BATCH_L(d.L, LMAXK, fp64::h_cell<LL>(M, a, i));
-      if (st == 2) check_finite_column(d.h, M.g.N, d.L, i, sc.status);
+      if (st == 2 && d.check) check_finite_column(d.h, M.g.N, d.L, i, sc.status);
     } else if (EXT && M.air) {
       ISW_BATCH_L(d.L, LMAXK, fp64::air_u_edge<LL>(M, a, i));
     } else {
@@ -260,6 +260,7 @@ struct BatchSlot {
 
 struct FastGroup {
   int begin = 0, count = 0, form = 0, cap = 0;   // its tiles [begin, begin + count), their form, the kernel's capacity
+  bool walls = false;                       // a stack of it has thin walls
   size_t smem = 0;
 };
 
@@ -311,6 +312,7 @@ struct isw_batch {
     int mode = 0, cells = 0, k = 0;
   };
   std::map<int, LevelLayout> levels;
+  bool check = true;                          // false: thicknesses are not looked at (a Layers' own batch with options)
   bool pdl = true;                            // programmatic dependent launch between phase kernels
   bool fast_grid = false;                     // untiled stacks' sub-steps: one cooperative launch per stage (k_fast_grid)
   int untiled_form[2] = {0, 0};               // per form (FP64, mixed): any untiled stack
@@ -509,7 +511,7 @@ isw_batch::LevelLayout level_layout(const isw_batch *b, const BatchSlot &sl) {
 }
 
 bool tiles_form(const isw_batch *b, const BatchSlot &sl) {
-  return sl.used && !sl.layers->d.air && !has_options(sl.layers->d) && level_layout(b, sl).mode != 1;
+  return sl.used && !sl.layers->d.air && level_layout(b, sl).mode != 1;
 }
 
 // Modelled time (us) of a stack's tile launches in one step at exchange interval k <= the probe's: per stage a fixed part
@@ -643,8 +645,9 @@ bool resident(isw_batch *b, const Tiling &t) {
         smax = std::max(smax, tiles_smem(tiles_for(b->slots[q].layers->grid, t.P[q], t.K[q])->host, b->slots[q].layers->d.L, f == 1));
       }
     if (count.empty()) continue;
-    for (int cap = 0; cap < 2; cap++) {
-      const void *fn = fast_tiles_kernel(t.bps, cap, f == 1);
+    for (int kind = 0; kind < 4; kind++) {
+      if (f == 1 && kind >= 2) break;          // (walls are the FP64 form's)
+      const void *fn = fast_tiles_kernel(t.bps, kind & 1, kind >= 2 ? 2 : f);
       // the kernel's limit is one setting for every batch: always the most a tile may ask for
       ISW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(t.bps == 2 ? SMEM_TWO : SMEM_ONE)));
       int per = 0;
@@ -686,7 +689,7 @@ void rebuild(isw_batch *b) {
   const int ngroups = kbest > 0 ? 1 + *std::max_element(best.group.begin(), best.group.end()) : 0;
   std::vector<std::vector<TileRef>> grefs(ngroups);
   std::vector<size_t> gsmem(ngroups, 0);
-  std::vector<int> gform(ngroups, 0), gcap(ngroups, 0);
+  std::vector<int> gform(ngroups, 0), gcap(ngroups, 0), gwalls(ngroups, 0);
   std::vector<std::shared_ptr<TileCache>> used_tiles;
   std::vector<std::pair<size_t, int>> gfirst;     // per tiled stack in order: its group, its first tile within the group
   for (auto &sl : b->slots) {
@@ -699,6 +702,7 @@ void rebuild(isw_batch *b) {
     if (d.M.air) any_air = 1;
     if (d.M.air || has_options(d.M)) any_ext = 1;
     if (d.M.ob) any_ob = 1;
+    d.check = b->check ? 1 : 0;
     d.dt = sl.dt;
     d.L = d.M.L;
     lmax = std::max(lmax, d.L);
@@ -731,6 +735,7 @@ void rebuild(isw_batch *b) {
       d.tiles = tiles_on_device(sl.layers->grid, tc.get());
       gsmem[g] = std::max(gsmem[g], tiles_smem(tc->host, d.L, form_of(sl) == 1));
       gform[g] = form_of(sl);
+      if (d.M.wall) gwalls[g] = 1;
       gcap[g] = std::max(gcap[g], tiles_cap(tc->host, best.K[q], best.bps));
       gfirst.emplace_back((size_t)g, (int)grefs[g].size());
       for (int p = 0; p < best.P[q]; p++) grefs[g].push_back(TileRef{s, p});
@@ -816,6 +821,7 @@ void rebuild(isw_batch *b) {
     fg.smem = gsmem[g];
     fg.form = gform[g];
     fg.cap = gcap[g];
+    fg.walls = gwalls[g] != 0;
     refs.insert(refs.end(), grefs[g].begin(), grefs[g].end());
     b->groups.push_back(fg);
   }
@@ -957,7 +963,7 @@ void launch_fast(isw_batch *b, cudaStream_t st, int stage, long long timeout_ns,
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    launch_fast_tiles(b->fast_bps, fg.cap, fg.form == 1, cfg, b->cur, b->d_refs + fg.begin, stage, b->flags, b->status, timeout_ns, fault_block);
+    launch_fast_tiles(b->fast_bps, fg.cap, fg.walls ? 2 : fg.form, cfg, b->cur, b->d_refs + fg.begin, stage, b->flags, b->status, timeout_ns, fault_block);
     if (fault_block >= 0) break;             // the failure test runs the first group only
   }
 }
@@ -1274,6 +1280,15 @@ int isw_batch_add_air(isw_batch *b, isw_layers *layers, isw_transport *tr, doubl
                       double *M, double *M1, double *const *tracers, int ntr, double dt, int nfast, int *slot) {
   return batch_add(b, layers, tr, h, u, Fm, theta, M, M1, tracers, ntr, dt, nfast, slot);
 }
+
+// (library side: handles.cuh)
+void isw_batch_set_check(isw_batch *b, int on) {
+  if (b->check == (on != 0)) return;
+  b->check = on != 0;
+  b->dirty = true;
+}
+
+int isw_batch_pending(const isw_batch *b) { return *(volatile int *)b->status_host; }
 
 int isw_batch_remove(isw_batch *b, int slot) {
   return guarded([&] {

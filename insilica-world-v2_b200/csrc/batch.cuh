@@ -32,6 +32,7 @@ struct StackDesc {
   double dt;
   int L, has_tr, tiled;
   int eg;                    // tracers of one thread of the transport's edge passes
+  int check;                 // the step's end looks for non-finite thicknesses
   int s_stage;               // the slow tendency stages its blocks' neighbour records in shared memory
   int n[3];
   double cdt[3], tau[3], inv_n[3];
@@ -241,11 +242,11 @@ const void *fast_grid_kernel_mixed();
 void launch_fast_grid_mixed(const cudaLaunchConfig_t &cfg, const StackDesc *desc, const Sched &sc, int stage, int nsub,
                             GridBarrier *bar, BatchStatus *status, long long timeout_ns);
 
-// The tiled fast loop (fast_tiles.cu): a form's kernel of a capacity for `bps` tile blocks per SM,
-// its block size, and its launch.
-const void *fast_tiles_kernel(int bps, int cap, bool mixed);
+// The tiled fast loop (fast_tiles.cu): the kernel of a form (0 FP64, 1 mixed, 2 FP64 with walls) and capacity
+// for `bps` tile blocks per SM, its block size, and its launch.
+const void *fast_tiles_kernel(int bps, int cap, int form);
 int fast_tiles_threads(int bps);
-void launch_fast_tiles(int bps, int cap, bool mixed, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
+void launch_fast_tiles(int bps, int cap, int form, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
                        unsigned *flags, BatchStatus *status, long long timeout_ns, int fault_block);
 
 }  // namespace bt

@@ -77,7 +77,10 @@ __device__ __forceinline__ double slot_flux(const double *fl, unsigned v) {
 }
 __device__ __forceinline__ float slot_flux(const float *fl, unsigned v) { return fl[v]; }
 
-template <int NT, int CAP>
+// Bit 15 of an edge's local cells: a thin wall closes it (tiles have at most 32000 cells).
+constexpr unsigned CLOSED = 0x8000u;
+
+template <int NT, int CAP, bool WALL>
 __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, unsigned *flags, BatchStatus *status,
                                           long long timeout_ns, bool skip, unsigned char *smem, const int *cnt) {
   constexpr int CM = TILE_CAP[CAP].C, EM = TILE_CAP[CAP].E, AM = TILE_CAP[CAP].A;
@@ -120,6 +123,7 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
         const double H = M.He[x[j].x], G = M.G[x[j].x];
         ub[j] = M.ub0[x[j].x];
         eid[e] = x[j].x;
+        if (WALL && M.wall && M.wall[x[j].x] == 0) ij[j] |= CLOSED;
         const double l = m[j].x * H;
         GD[e] = make_double2(G, m[j].y);
         lh[e] = l;
@@ -188,7 +192,7 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
 #pragma unroll
       for (int j = 0; j < EM; j++) {
         dy[j] = 0.0;
-        if (t + j * NT < en) dy[j] = -(Y[ij[j] >> 16] - Y[ij[j] & 0xffffu]);
+        if (t + j * NT < en) dy[j] = -(Y[ij[j] >> 16] - Y[ij[j] & 0x7fffu]);
       }
 #pragma unroll
       for (int j = 0; j < EM; j++) {
@@ -197,7 +201,8 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
           const double v = ub[j];
           const double2 gd = GD[e];
           if (j < AM && e < ering) acc[j < AM ? j : 0] += v;
-          const double nv = v + tau * (dy[j] / gd.y + gd.x);
+          double nv = v + tau * (dy[j] / gd.y + gd.x);
+          if (WALL && (ij[j] & CLOSED)) nv = 0.0;              // walls (its wind starts from zero, so its sum is zero too)
           ub[j] = nv;
           fl[e] = lh[e] * nv;
         }
@@ -248,7 +253,7 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
       }
 #pragma unroll
       for (int j = 0; j < AM; j++)
-        if (t + j * NT < ering) F[l * ering + t + j * NT] = he[j] * (us[j] - ubs[j]) + he[j] * acc[j];
+        if (t + j * NT < ering) F[l * ering + t + j * NT] = WALL && (ij[j] & CLOSED) ? 0.0 : he[j] * (us[j] - ubs[j]) + he[j] * acc[j];
     }
   }
   __syncthreads();
@@ -307,13 +312,13 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
       const int e = t + j * NT;
       if (e < ering) {
         double f = F[l * ering + e];
-        f *= sc[l * nc1 + (f > 0 ? ij[j] & 0xffffu : ij[j] >> 16)];
+        f *= sc[l * nc1 + (f > 0 ? ij[j] & 0x7fffu : ij[j] >> 16)];
         const double x = f * le[j];
         F[l * ering + e] = x;
         if (e < eown) {
           const size_t o = (size_t)l * E + eid[e];
           if (a.Fm) a.Fm[o] = x * a.dt;
-          a.un[o] = u0[j] + a.cdt * tp[j] + dub[j];
+          a.un[o] = WALL && (ij[j] & CLOSED) ? 0.0 : u0[j] + a.cdt * tp[j] + dub[j];
         }
       }
     }
@@ -339,7 +344,7 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
       }
     }
   }
-  if (st == 2 && !finite) raise_status(status, ISW_ENOTFINITE);
+  if (st == 2 && !finite && d.check) raise_status(status, ISW_ENOTFINITE);
 }
 
 // The mixed form: deviations deta = eta - eta0 and dub = ub - ub0 from zero in FP32, ub0's divergence c0 formed once per
@@ -634,7 +639,8 @@ __device__ __forceinline__ void tile_mixed(const StackDesc &d, int p, int st, un
   if (st == 2 && !finite) raise_status(status, ISW_ENOTFINITE);
 }
 
-template <int NT, int CAP, bool MIXED>
+// FORM: 0 FP64, 1 mixed, 2 FP64 with thin walls.
+template <int NT, int CAP, int FORM>
 __global__ void __launch_bounds__(NT, TILE_NT1 / NT) k_fast_tiles(const StackDesc *__restrict__ S, const TileRef *__restrict__ refs,
                                                               int st, unsigned *flags, BatchStatus *status, long long timeout_ns,
                                                               int fault_block) {
@@ -650,29 +656,31 @@ __global__ void __launch_bounds__(NT, TILE_NT1 / NT) k_fast_tiles(const StackDes
   __syncthreads();
   const bool skip = (int)blockIdx.x == fault_block;
   unsigned *own = flags + (size_t)d.tile_base * FLAG_STRIDE;
-  if (MIXED) tile_mixed<NT, CAP>(d, tr.p, st, own, status, timeout_ns, skip, smem, cnt);
-  else tile_fp64<NT, CAP>(d, tr.p, st, own, status, timeout_ns, skip, smem, cnt);
+  if (FORM == 1) tile_mixed<NT, CAP>(d, tr.p, st, own, status, timeout_ns, skip, smem, cnt);
+  else tile_fp64<NT, CAP, FORM == 2>(d, tr.p, st, own, status, timeout_ns, skip, smem, cnt);
 }
 
 using Kernel = void (*)(const StackDesc *, const TileRef *, int, unsigned *, BatchStatus *, long long, int);
 
-template <int CAP>
-Kernel kernel_for(int bps, bool mixed) {
-  if (bps == 2) return mixed ? k_fast_tiles<TILE_NT2, CAP, true> : k_fast_tiles<TILE_NT2, CAP, false>;
-  return mixed ? k_fast_tiles<TILE_NT1, CAP, true> : k_fast_tiles<TILE_NT1, CAP, false>;
+template <int NT, int CAP>
+Kernel kernel_for(int form) {
+  return form == 0 ? k_fast_tiles<NT, CAP, 0> : form == 1 ? k_fast_tiles<NT, CAP, 1> : k_fast_tiles<NT, CAP, 2>;
 }
 
-Kernel kernel_for(int bps, int cap, bool mixed) { return cap == 0 ? kernel_for<0>(bps, mixed) : kernel_for<1>(bps, mixed); }
+Kernel kernel_for(int bps, int cap, int form) {
+  if (bps == 2) return cap == 0 ? kernel_for<TILE_NT2, 0>(form) : kernel_for<TILE_NT2, 1>(form);
+  return cap == 0 ? kernel_for<TILE_NT1, 0>(form) : kernel_for<TILE_NT1, 1>(form);
+}
 
 }  // namespace
 
-const void *fast_tiles_kernel(int bps, int cap, bool mixed) { return (const void *)kernel_for(bps, cap, mixed); }
+const void *fast_tiles_kernel(int bps, int cap, int form) { return (const void *)kernel_for(bps, cap, form); }
 
 int fast_tiles_threads(int bps) { return bps == 2 ? TILE_NT2 : TILE_NT1; }
 
-void launch_fast_tiles(int bps, int cap, bool mixed, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
+void launch_fast_tiles(int bps, int cap, int form, const cudaLaunchConfig_t &cfg, const StackDesc *desc, const TileRef *refs, int stage,
                        unsigned *flags, BatchStatus *status, long long timeout_ns, int fault_block) {
-  ISW_CUDA(cudaLaunchKernelEx(&cfg, kernel_for(bps, cap, mixed), desc, refs, stage, flags, status, timeout_ns, fault_block));
+  ISW_CUDA(cudaLaunchKernelEx(&cfg, kernel_for(bps, cap, form), desc, refs, stage, flags, status, timeout_ns, fault_block));
 }
 
 }  // namespace bt

@@ -14,6 +14,8 @@ struct GraphEntry {
 };
 
 struct isw_batch;
+extern "C" void isw_batch_set_check(isw_batch *b, int on);   // whether its steps look for non-finite thicknesses (default 1)
+extern "C" int isw_batch_pending(const isw_batch *b);        // the status code its next step would be refused with
 
 struct isw_layers {
   isw_grid *grid;
@@ -26,8 +28,10 @@ struct isw_layers {
   int *nonfinite;
   double nu4dt = 0;                 // nu4 dt of the last step (the exchange books the step's nabla^4 loss as heat)
   int version = 0;                  // bumped when an option is set: batches holding the stack rebuild its descriptor
+  GraphEntry last_key{};            // option stacks: the arguments of the last direct step and the option version it saw
+  int last_version = -1;            // (a repeat of both steps through the private batch)
   bool percall = false;             // FP64: step with the per-call kernels instead of the private batch
-  // the mixed form steps call by call through a private one-stack batch (its step graph and tiles)
+  // the private one-stack batch (its step graph and tiles) that direct calls step through
   isw_batch *solo = nullptr;
   int solo_slot = -1;
   GraphEntry solo_key{};

@@ -468,18 +468,23 @@ void layers_destroy(isw_layers *s) {
   (void)cudaGetLastError();         // a failure while freeing must not surface in the caller's next call
 }
 
+bool same_call(const GraphEntry &k, const double *h, const double *u, const double *Fm, double dt, int nfast) {
+  return k.h == h && k.u == u && k.Fm == Fm && k.dt == dt && k.nfast == nfast;
+}
+
 // A step call by call through a private batch holding this one stack (rebuilt when the arrays, dt or nfast change): the
-// tiled fast loop and one graph per step. The mixed form always steps this way; the FP64 form does when the stack has
-// no air and no option branches, with bit-identical results.
-void layers_step_solo(isw_layers *s, double *h, double *u, double *Fm, double dt, int nfast, cudaStream_t st) {
+// tiled fast loop and one graph per step; bit-identical to the per-call kernels. The mixed form always steps this way;
+// layers_step says when the FP64 form does.
+void layers_step_solo(isw_layers *s, double *h, double *u, double *Fm, double dt, int nfast, bool check, cudaStream_t st) {
   auto ok = [](int rc) { if (rc != ISW_OK) fail(rc, isw_last_error()); };
   if (!s->solo) ok(isw_batch_create(s->grid->device, &s->solo));
+  isw_batch_set_check(s->solo, check ? 1 : 0);
   if (!Fm) {
     if (!s->solo_Fm) s->solo_Fm = dalloc(s, (size_t)s->d.L * s->d.g.E);
     Fm = s->solo_Fm;
   }
   GraphEntry &k = s->solo_key;
-  if (s->solo_slot < 0 || k.h != h || k.u != u || k.Fm != Fm || k.dt != dt || k.nfast != nfast) {
+  if (s->solo_slot < 0 || !same_call(k, h, u, Fm, dt, nfast)) {
     if (s->solo_slot >= 0) ok(isw_batch_remove(s->solo, s->solo_slot));
     s->solo_slot = -1;
     int slot = -1;
@@ -498,19 +503,28 @@ void layers_step(isw_layers *s, double *h, double *u, double *Fm, double *theta,
   if (!s->d.air && theta) fail(ISW_EINVAL, "layers.step: theta is for air layers");
   if (s->d.nu4 != 0) s->nu4dt = s->d.nu4 * dt;   // the step's nabla^4 loss, booked as heat by an air exchange
   if (s->d.precision == ISW_MIXED) {
-    layers_step_solo(s, h, u, Fm, dt, nfast, st);
+    layers_step_solo(s, h, u, Fm, dt, nfast, true, st);
     return;
   }
   const LayersDev &D = s->d;
-  if (!s->percall && !D.air && !D.wall && !D.ob && !(D.shelf > 0) && !D.sig && !D.tide && !D.cbot && !(D.cd_bot > 0)) {
+  if (!s->percall && !D.air) {
+    const bool options = D.wall || D.ob || D.shelf > 0 || D.sig || D.tide || D.cbot || D.cd_bot > 0;
     cudaStreamCaptureStatus cs0 = cudaStreamCaptureStatusNone;
     ISW_CUDA(cudaStreamIsCapturing(st, &cs0));
-    const GraphEntry &k = s->solo_key;
-    const bool ready = s->solo && s->solo_slot >= 0 && k.h == h && k.u == u && k.dt == dt && k.nfast == nfast &&
-                       (Fm ? k.Fm == Fm : k.Fm == s->solo_Fm);
+    const bool ready = s->solo && s->solo_slot >= 0 && same_call(s->solo_key, h, u, Fm ? Fm : s->solo_Fm, dt, nfast);
+    bool solo = cs0 == cudaStreamCaptureStatusNone || ready;
+    if (options) {
+      // option stacks: the private batch once a call repeats the one before it with no option set in between. Building it
+      // costs more than recording the per-call graph, of which eight are kept, so alternating arrays and options set before
+      // every step stay with the graphs. Never under a capture, nor while that batch would refuse to step.
+      solo = cs0 == cudaStreamCaptureStatusNone && s->last_version == s->version && same_call(s->last_key, h, u, Fm, dt, nfast) &&
+             !(s->solo && isw_batch_pending(s->solo));
+      s->last_key = GraphEntry{h, u, Fm, nullptr, dt, nfast, nullptr};
+      s->last_version = s->version;
+    }
     // (inside a capture of the caller's the batch cannot be built: the per-call kernels below give the same bits)
-    if (cs0 == cudaStreamCaptureStatusNone || ready) {
-      layers_step_solo(s, h, u, Fm, dt, nfast, st);
+    if (solo) {
+      layers_step_solo(s, h, u, Fm, dt, nfast, !options, st);
       return;
     }
   }

@@ -198,7 +198,7 @@ TileSetHost build_tiles(int N, int E, const int32_t *nbr, const int32_t *cellEdg
       if (o != p) { peers[p].insert(o); peers[o].insert(p); }
       auto a = lc.find(eI[e]), b = lc.find(eJ[e]);
       t.eix.push_back(e);
-      t.eix.push_back((int32_t)((a == lc.end() ? 0xffffu : (uint32_t)a->second) | (b == lc.end() ? 0xffffu : (uint32_t)b->second) << 16));
+      t.eix.push_back((int32_t)((a == lc.end() ? 0x7fffu : (uint32_t)a->second) | (b == lc.end() ? 0x7fffu : (uint32_t)b->second) << 16));
     }
     t.cell_off.push_back((int32_t)t.cells.size());
     t.edge_off.push_back((int32_t)t.edges.size());

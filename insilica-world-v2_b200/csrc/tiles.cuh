@@ -39,7 +39,7 @@ struct TileSetHost {
   // per local cell its six slots, 2 x local edge + (1 where the cell is the edge's eJ side), padded with 2 x the tile's
   // edges, and its global id as the last two halves of the 16-byte word: in cellEdge order and in ascending edge order
   std::vector<uint16_t> cedge, casc;
-  std::vector<int32_t> eix;                    // per local edge (global id, local cells eI | eJ << 16; 0xffff outside)
+  std::vector<int32_t> eix;                    // per local edge (global id, local cells eI | eJ << 16; 0x7fff outside)
   std::vector<int32_t> nbr_off, nbrs;          // per tile: the tiles it exchanges with (symmetric)
 };
 

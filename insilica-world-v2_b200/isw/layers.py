@@ -32,9 +32,9 @@ class Layers:
     def __init__(self, dg, layers=1, b=None, grav=GRAV, gprime=(), drag=0.0, stress=0.0, nu4=0.0, floor=1.0, rotation=1.0,
                  div_damp=DIV_DAMP, air=None, vmix=0.0, thin=2.0, wall=None, thin_wind=0.0, shelf=0.0, vmix_cd=0.0,
                  shelf_bed=False, batched=True, precision=None):
-        """The reference's constructor (layers.py:36-37). batched (this core's): FP64 Boussinesq layers without option
-        branches step through a private one-stack batch (tiled fast loop, one graph; bit-identical results); False keeps
-        the per-call kernels. precision (this core's): 'double' or 'mixed' for this object; None takes the grid's form
+        """The reference's constructor (layers.py:36-37). batched (this core's): FP64 Boussinesq layers step through
+        a private one-stack batch (tiled fast loop, one graph; bit-identical results), with option branches from the first
+        call that repeats the one before it; False keeps the per-call kernels. precision (this core's): 'double' or 'mixed' for this object; None takes the grid's form
         (the precision switch in force when the DeviceGrid was made)."""
         if precision not in (None, 'double', 'mixed'):
             raise ValueError(f'Layers: precision {precision!r}, want double or mixed')

@@ -1,0 +1,63 @@
+"""The step's routes for option stacks on a B200: through the private one-stack batch (its fast loop in tiles, walls
+included) from the first call that repeats the one before it, call by call otherwise; every mix equals the call-by-call
+kernels bit for bit."""
+from pathlib import Path
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+GOLDEN = Path(__file__).resolve().parent / 'golden'
+
+
+def T(a):
+    return torch.as_tensor(np.ascontiguousarray(a), dtype=torch.float64, device='cuda:0')
+
+
+def golden(name):
+    with np.load(GOLDEN / f'{name}.npz') as z:
+        return {k: z[k] for k in z.files}
+
+
+@pytest.mark.parametrize('options', ['all', 'walls', 'fields'])
+def test_option_routes_equal_per_call(grid4, options):
+    """Repeated calls, two sets of arrays in turn, an option set between calls, Fm given and not: h, u and Fm equal the
+    per-call kernels' after every step; a NaN thickness is stepped, not refused, as before."""
+    from isw.gpu import DeviceGrid
+    from isw.layers import Layers
+    z = golden('options_n4')
+    dg = DeviceGrid(grid4)
+    dt, nfast = float(z['dt']), int(z['nfast'])
+    cores = []
+    for batched in (True, False):
+        kw = dict(wall=z['wall']) if options != 'fields' else {}
+        if options == 'all':
+            kw.update(shelf=50.0, shelf_bed=True)
+        core = Layers(dg, 2, b=z['b'], gprime=[0.02], stress=[0.0, 2.5e-4], nu4=float(z['nu4']), floor=1.0, batched=batched, **kw)
+        if options != 'walls':
+            core.sig, core.cd_bot, core.cbot = T(z['sig']), 2.5e-3, T(z['cbot'])
+        cores.append(core)
+    wall = T(z['wall']) if options != 'fields' else 1.0
+    sets = [[dict(h=T(z['h0']) * s, u=T(z['u0']) * wall, Fm=torch.zeros_like(T(z['u0']))) for s in (1.0, 1.001)] for _ in cores]
+    order = [(0, True), (0, True), (0, True), (1, True), (0, True), (1, True), (1, True), (1, False), (1, False), (0, True),
+             (0, True)]
+    tide = T(np.linspace(-0.3, 0.3, dg.N))
+    for n, (which, with_fm) in enumerate(order):
+        for core, ss in zip(cores, sets):
+            if n in (3, 9):
+                core.tide = tide if n == 3 else None
+            a = ss[which]
+            core.step(a['h'], a['u'], dt, nfast, a['Fm'] if with_fm else None)
+        torch.cuda.synchronize()
+        for name in ('h', 'u', 'Fm'):
+            x, y = (ss[which][name] for ss in sets)
+            assert torch.equal(x, y), (n, name)
+    for ss in sets:
+        ss[0]['h'][0, 7] = float('nan')
+    for _ in range(3):
+        for core, ss in zip(cores, sets):
+            core.step(ss[0]['h'], ss[0]['u'], dt, nfast, ss[0]['Fm'])
+    torch.cuda.synchronize()
+    assert all(core.status() == 0 for core in cores)
+    assert torch.equal(*(torch.nan_to_num(ss[0]['h'], nan=-1.0) for ss in sets))
