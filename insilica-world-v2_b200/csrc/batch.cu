@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(THREADS) k_phase(const StackDesc *__restrict__
     const StageArgs a = stage_args(d, st);
     ISW_BATCH_L(d.L, LMAXK, fp64::stage_pk<LL>(d.M, ch.begin / THREADS, stg));
     __syncthreads();
-    if (i < ch.end) ISW_BATCH_L(d.L, LMAXK, (fp64::slow_edge<LL, EXT, true>(d.M, a.us, a.cdt, i, nullptr, stg)));
+    if (i < ch.end) ISW_BATCH_L(d.L, LMAXK, (fp64::slow_edge<LL, EXT, true>(d.M, a.cdt, i, nullptr, stg)));
     return;
   }
   if (i >= ch.end) return;
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(THREADS) k_phase(const StackDesc *__restrict__
     if (EXT && M.air) ISW_BATCH_L(d.L, LMAXK, fp64::air_fast_init_edge<LL>(M, a.u0, i));
   } else if (PH == PH_S) {
     const StageArgs a = stage_args(d, st);
-    ISW_BATCH_L(d.L, LMAXK, fp64::slow_edge<LL, EXT>(M, a.us, a.cdt, i, EXT && M.air ? d.theta : nullptr));
+    ISW_BATCH_L(d.L, LMAXK, fp64::slow_edge<LL, EXT>(M, a.cdt, i, EXT && M.air ? d.theta : nullptr));
   } else if (PH == PH_CS) {
     const StageArgs a = stage_args(d, st);
     if (EXT && M.air) ISW_BATCH_L(d.L, LMAXK, fp64::air_scale_cell<LL>(M, a, i));

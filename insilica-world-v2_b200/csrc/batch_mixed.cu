@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(THREADS) k_phase_m(const StackDesc *__restrict
     const mixed::MStageArgs a = mixed::mstage_args(d, st);
     ISW_BATCH_L(d.L, LMAXK, mixed::stage_pk4<LL>(d.M, ch.begin / THREADS, stg4));
     __syncthreads();
-    if (i < ch.end) ISW_BATCH_L(d.L, LMAXK, (mixed::slow_edge<LL, true>(d.M, a.us, a.cdt, i, stg4)));
+    if (i < ch.end) ISW_BATCH_L(d.L, LMAXK, (mixed::slow_edge<LL, true>(d.M, a.cdt, i, stg4)));
     return;
   }
   if (i >= ch.end) return;
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(THREADS) k_phase_m(const StackDesc *__restrict
     ISW_BATCH_L(d.L, LMAXK, mixed::edge_hq<LL>(M, a.hs, a.us, i));
   } else if (PH == PH_S) {
     const mixed::MStageArgs a = mixed::mstage_args(d, st);
-    ISW_BATCH_L(d.L, LMAXK, mixed::slow_edge<LL>(M, a.us, a.cdt, i));
+    ISW_BATCH_L(d.L, LMAXK, mixed::slow_edge<LL>(M, a.cdt, i));
   } else if (PH == PH_CS) {
     const mixed::MStageArgs a = mixed::mstage_args(d, st);
     ISW_BATCH_L(d.L, LMAXK, mixed::scale_sum_cell<LL>(M, a, i));

@@ -47,6 +47,11 @@ struct GridDev {
   // per cell, in ascending edge order (6 slots, pads -1): 2 x edge + (1 where the cell is the edge's eJ side), and the cell
   // on the edge's other side; what cellEdgeAsc with eI and eJ of every edge would say, in a quarter of the loads
   const int *ascE, *ascN;
+  const int4 *edge4;              // (eI, eJ, ev1, ev2) per edge, one 16-byte load
+  // per cell and slot (pads 0): sign l_e, and l_e d_e / 4, the kinetic energy's weight; read as rows of vectors in place of
+  // gathers of l_e and d_e through cellEdge
+  const double *cLe, *cKe;
+  const float *cLe32, *cKe32;
   const int8_t *cellSign, *vEdgeSign, *vSlot;
   const double *le, *de, *areaCell, *areaV, *fV, *kite, *w, *d2wt;
   const float *w32, *d2wt32, *le32, *de32, *rde32, *rle32, *rA32, *rAV32, *kite32;
@@ -69,6 +74,26 @@ __device__ __forceinline__ void slots6(const int *__restrict__ t, int i, int out
 #pragma unroll
   for (int q = 0; q < 3; q++) {
     const int2 v = p[q];
+    out[2 * q] = v.x;
+    out[2 * q + 1] = v.y;
+  }
+}
+
+__device__ __forceinline__ void slots6(const double *__restrict__ t, int i, double out[6]) {
+  const double2 *p = reinterpret_cast<const double2 *>(t + (size_t)i * 6);
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const double2 v = p[q];
+    out[2 * q] = v.x;
+    out[2 * q + 1] = v.y;
+  }
+}
+
+__device__ __forceinline__ void slots6(const float *__restrict__ t, int i, float out[6]) {
+  const float2 *p = reinterpret_cast<const float2 *>(t + (size_t)i * 6);
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const float2 v = p[q];
     out[2 * q] = v.x;
     out[2 * q + 1] = v.y;
   }

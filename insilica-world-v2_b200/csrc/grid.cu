@@ -185,6 +185,30 @@ static isw_grid *grid_create(const isw_grid_host *h, int device) {
       d.ascE = upload(g, ae.data(), ae.size());
       d.ascN = upload(g, an.data(), an.size());
     }
+    {
+      std::vector<int32_t> e4((size_t)E * 4);
+      for (int e = 0; e < E; e++) {
+        e4[4 * (size_t)e] = h->eI[e];
+        e4[4 * (size_t)e + 1] = h->eJ[e];
+        e4[4 * (size_t)e + 2] = h->ev1[e];
+        e4[4 * (size_t)e + 3] = h->ev2[e];
+      }
+      d.edge4 = reinterpret_cast<const int4 *>(upload(g, e4.data(), e4.size()));
+      std::vector<double> cl((size_t)N * 6, 0.0), ck((size_t)N * 6, 0.0);
+      std::vector<float> cl32((size_t)N * 6, 0.f), ck32((size_t)N * 6, 0.f);
+      for (size_t q = 0; q < (size_t)N * 6; q++) {
+        const int e = h->cellEdge[q];
+        if (e < 0) continue;
+        cl[q] = (double)h->cellSign[q] * h->le[e];
+        ck[q] = h->le[e] * h->de[e] * 0.25;
+        cl32[q] = (float)h->cellSign[q] * (float)h->le[e];
+        ck32[q] = (float)h->le[e] * (float)h->de[e] * 0.25f;
+      }
+      d.cLe = upload(g, cl.data(), cl.size());
+      d.cKe = upload(g, ck.data(), ck.size());
+      d.cLe32 = upload(g, cl32.data(), cl32.size());
+      d.cKe32 = upload(g, ck32.data(), ck32.size());
+    }
     d.nbr = upload(g, h->nbr, (size_t)N * 6);
     d.cellEdge = upload(g, h->cellEdge, (size_t)N * 6);
     d.cellEdgeAsc = upload(g, h->cellEdgeAsc, (size_t)N * 6);

@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(THREADS) k_stage_e(const LayersDev M, const St
 template <int L>
 __global__ void __launch_bounds__(THREADS) k_stage_s(const LayersDev M, const StageArgs a, const double *__restrict__ theta) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < M.g.E) fp64::slow_edge<L>(M, a.us, a.cdt, t, theta);
+  if (t < M.g.E) fp64::slow_edge<L>(M, a.cdt, t, theta);
 }
 
 // ---- air layers ----

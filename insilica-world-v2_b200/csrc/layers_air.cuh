@@ -75,11 +75,7 @@ __device__ __forceinline__ void air_bern_cell(const LayersDev &M, const double *
   int es[6];
   double kin[6];                             // l_e d_e / 4 of each slot
   slots6(g.cellEdge, i, es);
-#pragma unroll
-  for (int t = 0; t < 6; t++) {
-    const int e = es[t];
-    kin[t] = e >= 0 ? g.le[e] * g.de[e] * 0.25 : 0.0;
-  }
+  slots6(g.cKe, i, kin);
   const double area = g.areaCell[i];
 #pragma unroll
   for (int k = 0; k < L; k++) {
@@ -123,13 +119,7 @@ __device__ __forceinline__ void af_muphi_cell(const LayersDev &M, double tau, in
   int es[6];
   double flux_coef[6];                       // sign l_e of each slot
   slots6(g.cellEdge, i, es);
-  int sg[6];
-  signs6(g.cellSign, i, sg);
-#pragma unroll
-  for (int s = 0; s < 6; s++) {
-    const int e = es[s];
-    flux_coef[s] = e >= 0 ? (double)sg[s] * g.le[e] : 0.0;
-  }
+  slots6(g.cLe, i, flux_coef);
   const double area = g.areaCell[i];
   double fast_load[L];
   double above = 0;
@@ -157,7 +147,8 @@ template <int L>
 __device__ __forceinline__ void af_u_edge(const LayersDev &M, double tau, int e) {
   const GridDev &g = M.g;
   const int N = g.N, E = g.E;
-  const int a = g.eI[e], b = g.eJ[e];
+  const int2 ab = g.eIJ[e];
+  const int a = ab.x, b = ab.y;
   const double de = g.de[e], Ge = M.G[e];
 #pragma unroll
   for (int k = 0; k < L; k++) {

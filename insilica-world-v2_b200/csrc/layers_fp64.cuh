@@ -70,7 +70,8 @@ __device__ __forceinline__ void eta0_cell(const LayersDev &M, const double *__re
 template <int L, bool OPT = true>
 __device__ __forceinline__ void ubar0_edge(const LayersDev &M, const double *__restrict__ h, const double *__restrict__ u, int e) {
   const int N = M.g.N, E = M.g.E;
-  const int a = M.g.eI[e], b = M.g.eJ[e];
+  const int2 ab = M.g.eIJ[e];
+  const int a = ab.x, b = ab.y;
   double H = 0, U = 0;
 #pragma unroll
   for (int k = 0; k < L; k++) {
@@ -88,13 +89,7 @@ __device__ __forceinline__ void div_cell(const LayersDev &M, const double *__res
   int es[6];
   double c[6];
   slots6(g.cellEdge, i, es);
-  int sg[6];
-  signs6(g.cellSign, i, sg);
-#pragma unroll
-  for (int s = 0; s < 6; s++) {
-    const int e = es[s];
-    c[s] = e >= 0 ? (double)sg[s] * g.le[e] : 0.0;
-  }
+  slots6(g.cLe, i, c);
   const double A = g.areaCell[i];
 #pragma unroll
   for (int k = 0; k < L; k++) {
@@ -132,7 +127,8 @@ __device__ __forceinline__ void curl_vertex(const LayersDev &M, const double *__
 template <int L>
 __device__ __forceinline__ void lap_edge(const LayersDev &M, double *__restrict__ out, int e) {
   const GridDev &g = M.g;
-  const int a = g.eI[e], b = g.eJ[e], v1 = g.ev1[e], v2 = g.ev2[e];
+  const int4 x = g.edge4[e];
+  const int a = x.x, b = x.y, v1 = x.z, v2 = x.w;
   const double de = g.de[e], le = g.le[e];
 #pragma unroll
   for (int k = 0; k < L; k++) {
@@ -154,11 +150,7 @@ __device__ __forceinline__ void bern_cell(const LayersDev &M, const double *__re
   int es[6];
   double c[6];
   slots6(g.cellEdge, i, es);
-#pragma unroll
-  for (int t = 0; t < 6; t++) {
-    const int e = es[t];
-    c[t] = e >= 0 ? g.le[e] * g.de[e] * 0.25 : 0.0;
-  }
+  slots6(g.cKe, i, c);
   const double A = g.areaCell[i];
   double Mp = 0, P = 0;
 #pragma unroll
@@ -220,7 +212,8 @@ template <int L, bool OPT = true>
 __device__ __forceinline__ void edge_hq(const LayersDev &M, const double *__restrict__ h, const double *__restrict__ u, int e) {
   const GridDev &g = M.g;
   const int N = g.N, E = g.E, NV = g.NV;
-  const int a = g.eI[e], b = g.eJ[e], v1 = g.ev1[e], v2 = g.ev2[e];
+  const int4 x = g.edge4[e];
+  const int a = x.x, b = x.y, v1 = x.z, v2 = x.w;
   constexpr int PS = pk_stride(L);
   double r[PS];
   r[PS - 1] = 0.0;
@@ -258,19 +251,29 @@ __device__ __forceinline__ void stage_pk(const LayersDev &M, int c, double *stg)
 // STG: the neighbours' packed records come from `stg`, this block's staged copy of the distinct records its edges'
 // rows name (stage_pk), instead of from M.pk; the same values in the same order.
 template <int L, bool OPT = true, bool STG = false>
-__device__ __forceinline__ void slow_edge(const LayersDev &M, const double *__restrict__ u, double dts, int e,
+__device__ __forceinline__ void slow_edge(const LayersDev &M, double dts, int e,
                                           const double *__restrict__ theta = nullptr, const double *stg = nullptr) {
   const GridDev &g = M.g;
   const int N = g.N, E = g.E;
-  double he[L], cap[L], qf[L], Q[L];
+  double he[L], ue[L], cap[L], qf[L], Q[L];
   constexpr int PS = pk_stride(L);
-  const double *pe = M.pk + (size_t)e * PS;
+  {                                            // the edge's own packed record (which its neighbours gather too)
+    const double2 *pe = reinterpret_cast<const double2 *>(M.pk + (size_t)e * PS);
+    double r[PS];
 #pragma unroll
-  for (int k = 0; k < L; k++) {
-    he[k] = M.hedge[(size_t)k * E + e];
-    cap[k] = M.thin * he[k];
-    qf[k] = pe[k * 3 + 2];
-    Q[k] = 0;
+    for (int q = 0; q < PS / 2; q++) {
+      const double2 v = pe[q];
+      r[2 * q] = v.x;
+      r[2 * q + 1] = v.y;
+    }
+#pragma unroll
+    for (int k = 0; k < L; k++) {
+      he[k] = r[k * 3 + 0];
+      ue[k] = r[k * 3 + 1];
+      qf[k] = r[k * 3 + 2];
+      cap[k] = M.thin * he[k];
+      Q[k] = 0;
+    }
   }
   // the row's neighbour ids and weights first (at most EOE_MAX, validated with the grid), then the gathers, all in
   // flight together; the sum runs in row order as the reference's loop does
@@ -304,13 +307,13 @@ __device__ __forceinline__ void slow_edge(const LayersDev &M, const double *__re
       }
     }
   }
-  const int a = g.eI[e], b = g.eJ[e];
+  const int2 ab = g.eIJ[e];
+  const int a = ab.x, b = ab.y;
   const double de = g.de[e];
   double T[L], sqk[L];
   double H = 0, U = 0, GT = 0;
 #pragma unroll
   for (int k = 0; k < L; k++) {
-    const double ue = u[(size_t)k * E + e];
     const double *Bl = M.B + (size_t)k * N;
     // a layer squeezed by the shelf fades its pressure force and takes a day's drag (reference layers.cu:293-297);
     // shelf off: sq = 1, the force is -(B_J - B_I) / d and the drag term (1 - 1) / 21600 = 0
@@ -318,7 +321,7 @@ __device__ __forceinline__ void slow_edge(const LayersDev &M, const double *__re
     const double sq0 = shk > 0 && he[k] < shk ? (he[k] - 2 * M.floor_ > 0 ? (he[k] - 2 * M.floor_) / (shk - 2 * M.floor_) : 0.0) : 1.0;
     const double sq = theta ? 1.0 : sq0;
     sqk[k] = sq0;
-    double d = Q[k] - (sq * (Bl[b] - Bl[a])) / de - (M.drag[k] + (1 - sq) / 21600.0) * ue;
+    double d = Q[k] - (sq * (Bl[b] - Bl[a])) / de - (M.drag[k] + (1 - sq) / 21600.0) * ue[k];
     double ck = M.stress[k];
     if (OPT && k == L - 1 && (M.cd_bot > 0 || M.cbot)) {
       // the bottom layer's quadratic stress cd |u| (|u| from the normal and the TRiSK tangential wind) and the internal
@@ -326,13 +329,13 @@ __device__ __forceinline__ void slow_edge(const LayersDev &M, const double *__re
       if (M.cd_bot > 0) {
         double vt = 0;
         for (int t = 0; t < cnt; t++) vt += wv[t] * (STG ? stg : M.pk)[(size_t)ix[t] * PS + k * 3 + 1];
-        ck += M.cd_bot * sqrt(ue * ue + vt * vt);
+        ck += M.cd_bot * sqrt(ue[k] * ue[k] + vt * vt);
       }
       if (M.cbot) ck += M.cbot[e];
     }
     if (ck != 0) {
       const double r = ck / (he[k] > M.floor_ ? he[k] : M.floor_);
-      d = d - ((r * dts > 1e-8) ? (1 - exp(-r * dts)) / dts : r) * ue;
+      d = d - ((r * dts > 1e-8) ? (1 - exp(-r * dts)) / dts : r) * ue[k];
     }
     if (theta) {                   // air layers: + pibar grad(theta) (reference layers.cu:322-326)
       const double *tl = theta + (size_t)k * N;
@@ -347,7 +350,7 @@ __device__ __forceinline__ void slow_edge(const LayersDev &M, const double *__re
     if (M.nu4 != 0) d = d - M.nu4 * M.L2[(size_t)k * E + e];
     T[k] = d;
     H += he[k];
-    U += he[k] * ue;
+    U += he[k] * ue[k];
   }
   if (OPT && theta && M.shelf > 0) {   // air squeezed against the ground takes its neighbours' tendency (layers.cu:341-355)
     double Tn[L];
@@ -667,15 +670,14 @@ __device__ __forceinline__ void h_cell(const LayersDev &M, const StageArgs &a, i
   for (int k = 0; k < L; k++) div[k] = 0;
   int es[6];
   slots6(g.cellEdge, i, es);
-  int sg[6];
-  signs6(g.cellSign, i, sg);
+  double c[6];
+  slots6(g.cLe, i, c);
 #pragma unroll
   for (int s = 0; s < 6; s++) {
     const int e = es[s];
     if (e < 0) continue;
-    const double c = (double)sg[s] * g.le[e];
 #pragma unroll
-    for (int k = 0; k < L; k++) div[k] += c * limited(M, k, e);
+    for (int k = 0; k < L; k++) div[k] += c[s] * limited(M, k, e);
   }
   const double A = g.areaCell[i];
 #pragma unroll
@@ -704,7 +706,8 @@ template <int L, bool OPT = true>
 __device__ __forceinline__ void vmix_edge(const LayersDev &M, const double *__restrict__ h, double *__restrict__ u, double dt, int e) {
   const GridDev &g = M.g;
   const int N = g.N, E = g.E;
-  const int ia = g.eI[e], ib = g.eJ[e];
+  const int2 ab = g.eIJ[e];
+  const int ia = ab.x, ib = ab.y;
   const double c = M.vmix, cd = M.vmix_cd;
   double d = 0;
 #pragma unroll

@@ -34,7 +34,8 @@ struct MStageArgs {
 template <int L>
 __device__ __forceinline__ void ubar0_edge(const LayersDev &M, const double *__restrict__ h, const double *__restrict__ u, int e) {
   const int N = M.g.N, E = M.g.E;
-  const int a = M.g.eI[e], b = M.g.eJ[e];
+  const int2 ab = M.g.eIJ[e];
+  const int a = ab.x, b = ab.y;
   double H = 0, U = 0;
 #pragma unroll
   for (int k = 0; k < L; k++) {
@@ -53,13 +54,7 @@ __device__ __forceinline__ void div_cell(const LayersDev &M, const T *__restrict
   int es[6];
   float c[6];
   slots6(g.cellEdge, i, es);
-  int sg[6];
-  signs6(g.cellSign, i, sg);
-#pragma unroll
-  for (int s = 0; s < 6; s++) {
-    const int e = es[s];
-    c[s] = e >= 0 ? (float)sg[s] * g.le32[e] : 0.f;
-  }
+  slots6(g.cLe32, i, c);
   const float rA = g.rA32[i];
 #pragma unroll
   for (int k = 0; k < L; k++) {
@@ -97,7 +92,8 @@ __device__ __forceinline__ void curl_vertex(const LayersDev &M, const T *__restr
 template <int L>
 __device__ __forceinline__ void lap_edge(const LayersDev &M, float *__restrict__ out, int e) {
   const GridDev &g = M.g;
-  const int a = g.eI[e], b = g.eJ[e], v1 = g.ev1[e], v2 = g.ev2[e];
+  const int4 x = g.edge4[e];
+  const int a = x.x, b = x.y, v1 = x.z, v2 = x.w;
   const float rde = g.rde32[e], rle = g.rle32[e];
 #pragma unroll
   for (int k = 0; k < L; k++) {
@@ -119,11 +115,7 @@ __device__ __forceinline__ void bern_cell(const LayersDev &M, const double *__re
   int es[6];
   float c[6];
   slots6(g.cellEdge, i, es);
-#pragma unroll
-  for (int t = 0; t < 6; t++) {
-    const int e = es[t];
-    c[t] = e >= 0 ? g.le32[e] * g.de32[e] * 0.25f : 0.f;
-  }
+  slots6(g.cKe32, i, c);
   const float rA = g.rA32[i];
   double Mp = 0;
 #pragma unroll
@@ -176,7 +168,8 @@ template <int L>
 __device__ __forceinline__ void edge_hq(const LayersDev &M, const double *__restrict__ h, const float *__restrict__ u, int e) {
   const GridDev &g = M.g;
   const int N = g.N, E = g.E, NV = g.NV;
-  const int a = g.eI[e], b = g.eJ[e], v1 = g.ev1[e], v2 = g.ev2[e];
+  const int4 x = g.edge4[e];
+  const int a = x.x, b = x.y, v1 = x.z, v2 = x.w;
   float4 *pp = M.pk4 + (size_t)e * L;
 #pragma unroll
   for (int k = 0; k < L; k++) {
@@ -202,17 +195,18 @@ __device__ __forceinline__ void stage_pk4(const LayersDev &M, int c, float4 *stg
 
 // STG: the neighbours' records come from `stg` (stage_pk4) instead of M.pk4; the same values in the same order.
 template <int L, bool STG = false>
-__device__ __forceinline__ void slow_edge(const LayersDev &M, const float *__restrict__ u, double dts, int e,
+__device__ __forceinline__ void slow_edge(const LayersDev &M, double dts, int e,
                                           const float4 *stg = nullptr) {
   const GridDev &g = M.g;
   const int N = g.N, E = g.E;
-  float he[L], cap[L], qf[L], Q[L];
+  float he[L], ue[L], cap[L], qf[L], Q[L];
   const float thin = (float)M.thin;
   const float4 *pe = M.pk4 + (size_t)e * L;
 #pragma unroll
   for (int k = 0; k < L; k++) {
     const float4 p = pe[k];
     he[k] = p.x;
+    ue[k] = p.y;
     cap[k] = thin * p.x;
     qf[k] = p.z;
     Q[k] = 0.f;
@@ -238,26 +232,26 @@ __device__ __forceinline__ void slow_edge(const LayersDev &M, const float *__res
       }
     }
   }
-  const int a = g.eI[e], b = g.eJ[e];
+  const int2 ab = g.eIJ[e];
+  const int a = ab.x, b = ab.y;
   const double rde = g.rde[e];
   const float fdts = (float)dts, flo = (float)M.floor_, nu4 = (float)M.nu4;
   float T[L];
   float H = 0, U = 0, GT = 0;
 #pragma unroll
   for (int k = 0; k < L; k++) {
-    const float ue = u[(size_t)k * E + e];
     const double *Bl = M.B + (size_t)k * N;
-    float d = Q[k] - (float)((Bl[b] - Bl[a]) * rde) - (float)M.drag[k] * ue;
+    float d = Q[k] - (float)((Bl[b] - Bl[a]) * rde) - (float)M.drag[k] * ue[k];
     const float ck = (float)M.stress[k];
     if (ck != 0.f) {
       const float r = ck / fmaxf(he[k], flo);
       const float rd = r * fdts;
-      d -= (rd > 1e-8f ? -expm1f(-rd) / fdts : r) * ue;     // exact exponential decay over the stage
+      d -= (rd > 1e-8f ? -expm1f(-rd) / fdts : r) * ue[k];     // exact exponential decay over the stage
     }
     if (nu4 != 0.f) d -= nu4 * M.L2f[(size_t)k * E + e];
     T[k] = d;
     H += he[k];
-    U += he[k] * ue;
+    U += he[k] * ue[k];
   }
 #pragma unroll
   for (int k = 0; k < L; k++) GT += he[k] * T[k];
@@ -530,15 +524,14 @@ __device__ __forceinline__ void h_cell(const LayersDev &M, const MStageArgs &a, 
   for (int k = 0; k < L; k++) div[k] = 0;
   int es[6];
   slots6(g.cellEdge, i, es);
-  int sg[6];
-  signs6(g.cellSign, i, sg);
+  double c[6];
+  slots6(g.cLe, i, c);
 #pragma unroll
   for (int s = 0; s < 6; s++) {
     const int e = es[s];
     if (e < 0) continue;
-    const double c = (double)sg[s] * g.le[e];
 #pragma unroll
-    for (int k = 0; k < L; k++) div[k] += c * limited(M, k, e);
+    for (int k = 0; k < L; k++) div[k] += c[s] * limited(M, k, e);
   }
   const double rA = g.rA[i];
 #pragma unroll
