@@ -238,13 +238,13 @@ int isw_batch_flush(isw_batch *b, void *stream);
 /* The batch's layout: registered stacks, fast-loop tiles, the exchange interval in use, the largest tile's shared memory
  * (bytes), the cooperative launches per stage, tile blocks per SM (0 when untiled). */
 int isw_batch_info(isw_batch *b, int *stacks, int *tiles, int *tile_k, long long *smem_bytes, int *groups, int *blocks_per_sm);
-/* The batch's device status word: ISW_OK, ISW_ETIMEOUT after a grid barrier's bounded wait ran out, or ISW_ENOTFINITE
+/* The batch's device status word: ISW_OK, ISW_ETIMEOUT after a bounded wait of its kernels ran out, or ISW_ENOTFINITE
  * after a step left a NaN or Inf thickness (checked for every cell and layer at the end of each step). The kernel that
  * records a failure also writes it to a mapped host word, and isw_batch_step refuses to run (returning that status)
  * until the word is cleared, so later steps never run on a half-updated state. Synchronises `stream`; reset != 0
  * clears the word (restore the state first). */
 int isw_batch_status(isw_batch *b, void *stream, int reset);
-/* Failure-detection test: one step in which block 0 never arrives at the first grid barrier, so every other block's
+/* Failure-detection test: the first stage's tile launch with a tile that never raises its flag, so its neighbours'
  * bounded wait runs out after timeout_ns (1 ms .. 2 s) and the status word becomes ISW_ETIMEOUT. Test use only. */
 int isw_batch_fault_test(isw_batch *b, long long timeout_ns, void *stream);
 

@@ -3,20 +3,20 @@
 //
 // Each phase is one kernel over every stack at once: a table of chunks (stack, up to 256 items of its cells, edges,
 // vertices or tracer rows), one chunk per block, the stack's descriptor staged in shared memory. Stacks may sit on
-// different grids and have different layer counts. The barotropic fast loop of a stage is one cooperative kernel over
-// shared-memory tiles (tiles.cuh): k sub-steps per grid-wide exchange instead of two launches per sub-step; stacks
-// whose tiles would not fit in shared memory take the sub-steps as grid-wide kernels instead. The phase functions are
-// the per-call path's (layers_fp64.cuh, transport_fp64.cuh), so every stack's result is bit-identical to stepping it
-// alone, whatever else shares the launches.
+// different grids and have different layer counts. The barotropic fast loop of a stage and the stage's end are one
+// cooperative kernel over tiles per precision form (fast_tiles.cu): k sub-steps per exchange between neighbouring tiles
+// instead of two launches per sub-step; stacks whose tiles would not fit on chip take the sub-steps, the limiter and the
+// stage's end as grid-wide kernels. The phase functions are the per-call path's (layers_fp64.cuh, transport_fp64.cuh), so
+// every stack's result is bit-identical to stepping it alone, whatever else shares the launches.
 //
-// Per step: init (+ first Laplacian pass) | lap e | lap cv | lap e | per stage: A, E, S, fast loop, C, D |
+// Per step: init (+ first Laplacian pass) | lap e | lap cv | lap e | per stage: A, E, S, tiles (untiled: sub-steps, CS, D) |
 // vmix + FCT stage-1 edge fluxes | P1 (receiving masses, td, p1) | P2E | P2 | P3E | P3 | P4 (and M <- M1).
 //
-// The tile kernel's grid barrier waits with an iteration-bounded, time-bounded spin (globaltimer): if a wait runs out
-// it records ISW_ETIMEOUT in the batch's status word and every block returns. Phase D of the last stage checks every
-// new thickness and records ISW_ENOTFINITE for a NaN or Inf. The kernel that records a failure also writes it to a
-// mapped host word, and isw_batch_step refuses to run while that word is set (until isw_batch_status resets it), so a
-// caller that never polls cannot step on a half-updated state.
+// The tile kernel's waits (and the persistent grid-wide loop's barrier) are iteration-bounded, time-bounded spins
+// (globaltimer): if a wait runs out it records ISW_ETIMEOUT in the batch's status word and every block returns. The last
+// stage's end checks every new thickness and records ISW_ENOTFINITE for a NaN or Inf. The kernel that records a failure also
+// writes it to a mapped host word, and isw_batch_step refuses to run while that word is set (until isw_batch_status resets
+// it), so a caller that never polls cannot step on a half-updated state.
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -160,13 +160,15 @@ __global__ void __launch_bounds__(THREADS) k_phase(const StackDesc *__restrict__
       const EdgeRow r = edge_row(d, i);
     ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
     }
-  } else if (PH == PH_P1) {
-    ISW_BATCH_L(d.L, LMAXK, fp64::tr_c1<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
+  } else if (PH == PH_P1 || PH == PH_P1G) {
+    const CellRow r = cell_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, (fp64::tr_c1<LL, phase_tracers<PH>()>(d.T, d.tr, r.j0, r.n, r.c)));
   } else if (PH == PH_P2E) {
     const EdgeRow r = edge_row(d, i);
     ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 2, r.j0, r.j1, r.e));
-  } else if (PH == PH_P2) {
-    ISW_BATCH_L(d.L, LMAXK, fp64::tr_c2<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
+  } else if (PH == PH_P2 || PH == PH_P2G) {
+    const CellRow r = cell_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, (fp64::tr_c2<LL, phase_tracers<PH>()>(d.T, d.tr, r.j0, r.n, r.c)));
   } else if (PH == PH_P3E) {
     const EdgeRow r = edge_row(d, i);
     ISW_BATCH_L(d.L, LMAXK, fp64::tr_a_edge<LL>(d.T, d.tr, r.j0, r.j1, r.e));
@@ -315,6 +317,7 @@ struct isw_batch {
   bool check = true;                          // false: thicknesses are not looked at (a Layers' own batch with options)
   bool pdl = true;                            // programmatic dependent launch between phase kernels
   bool fast_grid = false;                     // untiled stacks' sub-steps: one cooperative launch per stage (k_fast_grid)
+  int cell_tracers[2] = {1, 1};               // per form: tracers of one thread of the first two cell passes (mixed: one)
   int untiled_form[2] = {0, 0};               // per form (FP64, mixed): any untiled stack
   size_t s_smem[2] = {0, 0};                  // per form: dynamic shared memory of the slow-tendency launch (staging)
   int grid_blocks[2] = {0, 0};                // per form: co-resident blocks of the cooperative grid-wide fast loop
@@ -661,16 +664,22 @@ bool resident(isw_batch *b, const Tiling &t) {
 
 void rebuild(isw_batch *b) {
   std::vector<StackDesc> desc;
-  std::vector<Chunk> cell[2], edge[2], vert[2], rows[2], erows[2];      // per form: [0] FP64 stacks, [1] mixed
+  std::vector<Chunk> cell[2], edge[2], vert[2], rows[2], erows[2], grows[2];      // per form: [0] FP64 stacks, [1] mixed
   std::vector<Chunk> wcell[2], wedge[2], uedge[2];                      // the untiled stacks': the sub-step passes' wide chunks, plain edges
   int nsub[3] = {0, 0, 0};
   int any_nu4 = 0, any_vmix = 0, any_tr = 0, any_untiled = 0, any_air = 0, any_ext = 0, any_ob = 0, lmax = 1;
   int untiled[2] = {0, 0};
   size_t s_smem[2] = {0, 0};
   const double cs[3] = {1.0 / 3.0, 1.0 / 2.0, 1.0};
-  long long edge_items[2] = {0, 0};                                     // per form: (tracer, edge) pairs
+  int most_layers = 1;                                                  // over both forms: the phase kernels' L
   for (auto &sl : b->slots)
-    if (sl.used && sl.tr) edge_items[form_of(sl)] += (long long)sl.ntr * sl.layers->grid->d.E;
+    if (sl.used) most_layers = std::max(most_layers, sl.layers->d.L);
+  long long edge_items[2] = {0, 0}, cell_items[2] = {0, 0};             // per form: (tracer, edge) and (tracer, cell) pairs
+  for (auto &sl : b->slots)
+    if (sl.used && sl.tr) {
+      edge_items[form_of(sl)] += (long long)sl.ntr * sl.layers->grid->d.E;
+      cell_items[form_of(sl)] += (long long)sl.ntr * sl.layers->grid->d.N;
+    }
   int used = 0;
   for (auto &sl : b->slots) used += sl.used ? 1 : 0;
   Tiling best;
@@ -762,7 +771,9 @@ void rebuild(isw_batch *b) {
       chunks(uedge[f], d.M.g.E);
     }
     if (d.has_tr) chunks(rows[f], sl.ntr * d.M.g.N);       // (tracer, cell) pairs
-    if (d.has_tr) {                                        // (tracers of a thread, edge)
+    if (d.has_tr) {                                        // (tracers of a thread, cell), (tracers of a thread, edge)
+      d.cg = f == 0 ? fp64::cell_tracers(cell_items[0], most_layers) : 1;
+      chunks(grows[f], (sl.ntr + d.cg - 1) / d.cg * d.M.g.N);
       d.eg = fp64::tracers_a_thread(edge_items[f], sl.ntr);
       chunks(erows[f], (sl.ntr + d.eg - 1) / d.eg * d.M.g.E);
     }
@@ -806,6 +817,7 @@ void rebuild(isw_batch *b) {
     all.insert(all.end(), vert[f].begin(), vert[f].end());
     all.insert(all.end(), rows[f].begin(), rows[f].end());
     all.insert(all.end(), erows[f].begin(), erows[f].end());
+    all.insert(all.end(), grows[f].begin(), grows[f].end());
     all.insert(all.end(), wcell[f].begin(), wcell[f].end());
     all.insert(all.end(), wedge[f].begin(), wedge[f].end());
     all.insert(all.end(), uedge[f].begin(), uedge[f].end());
@@ -871,7 +883,9 @@ void rebuild(isw_batch *b) {
     sc.nrows = (int)rows[f].size();
     sc.erows = sc.rows + sc.nrows;
     sc.nerows = (int)erows[f].size();
-    sc.wcell = sc.erows + sc.nerows;
+    sc.grows = sc.erows + sc.nerows;
+    sc.ngrows = (int)grows[f].size();
+    sc.wcell = sc.grows + sc.ngrows;
     sc.nwcell = (int)wcell[f].size();
     sc.wedge = sc.wcell + sc.nwcell;
     sc.nwedge = (int)wedge[f].size();
@@ -893,6 +907,7 @@ void rebuild(isw_batch *b) {
   b->any_ext = any_ext;
   b->any_ob = any_ob;
   b->lmax = kernel_lmax(lmax);
+  b->cell_tracers[0] = fp64::cell_tracers(cell_items[0], most_layers);
   b->s_smem[0] = s_smem[0];
   b->s_smem[1] = s_smem[1];
   if (s_smem[0] > 48 * 1024)
@@ -913,39 +928,47 @@ void rebuild(isw_batch *b) {
   }
 }
 
-// A phase over every stack: one kernel per precision form present (the FP64 stacks' first). pdl: the first of them is
-// launched as a programmatic dependent of the kernel before it in the stream (never directly after a cooperative tile
-// launch, which keeps plain stream order); a second one always is.
+// A phase over the stacks of form f.
 template <int PH>
+void launch_form(isw_batch *b, cudaStream_t st, int f, int stage, int j, bool pdl) {
+  const Sched &sc = b->scf[f];
+  const int nb = phase_blocks<PH>(sc);
+  if (!b->cur) fail(ISW_EINVAL, "batch: no stack descriptors selected for the launch");
+  if (f == 1) {
+    launch_phase_mixed(PH, b->lmax, nb, st, pdl, PH == PH_S ? b->s_smem[1] : 0, b->cur, sc, stage, j);
+    return;
+  }
+  const size_t smem = PH == PH_S ? b->s_smem[0] : 0;
+  if (b->any_ext) {
+    switch (b->lmax) {
+      case 2: launch_kernel(k_phase<PH, 2, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+      case 3: launch_kernel(k_phase<PH, 3, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+      case 5: launch_kernel(k_phase<PH, 5, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+      default: launch_kernel(k_phase<PH, 8, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+    }
+  } else {
+    switch (b->lmax) {
+      case 2: launch_kernel(k_phase<PH, 2, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+      case 3: launch_kernel(k_phase<PH, 3, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+      case 5: launch_kernel(k_phase<PH, 5, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+      default: launch_kernel(k_phase<PH, 8, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+    }
+  }
+}
+
+// A phase over every stack: one kernel per precision form present (the FP64 stacks' first); PHG in its place for a form
+// whose cell passes take several tracers a thread. pdl: the first of them is launched as a programmatic dependent of the
+// kernel before it in the stream (never directly after a cooperative tile launch, which keeps plain stream order); a
+// second one always is.
+template <int PH, int PHG = PH>
 void launch_phase(isw_batch *b, cudaStream_t st, int stage, int j, bool pdl = true) {
   bool first = true;
   for (int f = 0; f < 2; f++) {
-    const Sched &sc = b->scf[f];
-    const int nb = phase_blocks<PH>(sc);
-    if (nb == 0) continue;
-    if (!b->cur) fail(ISW_EINVAL, "batch: no stack descriptors selected for the launch");
+    if (phase_blocks<PH>(b->scf[f]) == 0) continue;
     const bool p = (first ? pdl : true) && b->pdl;
     first = false;
-    if (f == 1) {
-      launch_phase_mixed(PH, b->lmax, nb, st, p, PH == PH_S ? b->s_smem[1] : 0, b->cur, sc, stage, j);
-      continue;
-    }
-    const size_t smem = PH == PH_S ? b->s_smem[0] : 0;
-    if (b->any_ext) {
-      switch (b->lmax) {
-        case 2: launch_kernel(k_phase<PH, 2, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        case 3: launch_kernel(k_phase<PH, 3, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        case 5: launch_kernel(k_phase<PH, 5, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        default: launch_kernel(k_phase<PH, 8, true>, nb, st, p, smem, b->cur, sc, stage, j); break;
-      }
-    } else {
-      switch (b->lmax) {
-        case 2: launch_kernel(k_phase<PH, 2, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        case 3: launch_kernel(k_phase<PH, 3, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        case 5: launch_kernel(k_phase<PH, 5, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
-        default: launch_kernel(k_phase<PH, 8, false>, nb, st, p, smem, b->cur, sc, stage, j); break;
-      }
-    }
+    if (PHG != PH && b->cell_tracers[f] > 1) launch_form<PHG>(b, st, f, stage, j, p);
+    else launch_form<PH>(b, st, f, stage, j, p);
   }
 }
 
@@ -1033,9 +1056,9 @@ bool enqueue_dyn(isw_batch *b, cudaStream_t st) {
 
 // The transport passes after the stage-1 edge fluxes (P1 .. P4, M <- M1).
 void enqueue_tr_tail(isw_batch *b, cudaStream_t st) {
-  launch_phase<PH_P1>(b, st, 0, 0);
+  launch_phase<PH_P1, PH_P1G>(b, st, 0, 0);
   launch_phase<PH_P2E>(b, st, 0, 0);
-  launch_phase<PH_P2>(b, st, 0, 0);
+  launch_phase<PH_P2, PH_P2G>(b, st, 0, 0);
   launch_phase<PH_P3E>(b, st, 0, 0);
   launch_phase<PH_P3>(b, st, 0, 0);
   launch_phase<PH_P4>(b, st, 0, 0);
@@ -1363,7 +1386,7 @@ int isw_batch_step(isw_batch *b, void *stream) {
     if (!b) fail(ISW_EINVAL, "batch.step: null handle");
     const int code = *(volatile int *)b->status_host;
     if (code == ISW_ETIMEOUT)
-      fail(code, "batch.step: refused: an earlier step's grid barrier timed out, so the state is half-updated; restore "
+      fail(code, "batch.step: refused: an earlier step's wait on the device timed out, so the state is half-updated; restore "
                  "it and clear the status (isw_batch_status with reset) to step again");
     if (code != ISW_OK)
       fail(code, "batch.step: refused: an earlier step left a non-finite thickness; restore the state and clear the status "

@@ -1,6 +1,6 @@
 // Definitions shared by the batched step's translation units (batch.cu: plain FP64 phases and the step's host side;
 // batch_mixed.cu: the mixed form's phases, compiled with fused multiply-adds): the stack descriptor, chunk tables,
-// tiles, the bounded grid barrier, the phase list.
+// tiles, the bounded grid barrier of the persistent loop, the phase list.
 #pragma once
 #include <cuda/atomic>
 
@@ -31,7 +31,7 @@ struct StackDesc {
   double *theta;             // air layers: potential temperature (L x N); null for Boussinesq layers
   double dt;
   int L, has_tr, tiled;
-  int eg;                    // tracers of one thread of the transport's edge passes
+  int eg, cg;                // tracers of one thread of the transport's edge passes, of its first two cell passes
   int check;                 // the step's end looks for non-finite thicknesses
   int s_stage;               // the slow tendency stages its blocks' neighbour records in shared memory
   int n[3];
@@ -65,8 +65,9 @@ __device__ __forceinline__ void raise_status(BatchStatus *s, int code) {
 }
 
 struct Sched {
-  const Chunk *cell, *edge, *vert, *rows, *erows;   // rows: (tracer, cell) pairs; erows: (tracer, edge) pairs
-  int ncell, nedge, nvert, nrows, nerows;
+  const Chunk *cell, *edge, *vert, *rows, *erows;   // rows: (tracer, cell) pairs; erows: (tracers of a thread, edge)
+  const Chunk *grows;                               // (tracers of a thread, cell)
+  int ncell, nedge, nvert, nrows, nerows, ngrows;
   const Chunk *wcell, *wedge, *uedge;               // untiled stacks only: the sub-step passes' chunks (SUB_W... x THREADS),
   int nwcell, nwedge, nuedge;                       // and their edges in plain chunks
   BatchStatus *status;
@@ -174,8 +175,9 @@ __device__ __forceinline__ const StackDesc &stage_desc(const StackDesc *S, int s
 // a batch with air stacks runs VMIX, VHEAT (cells: the stress's heat back to theta) and HF1 in place of POST.
 // PH_ETA / PH_UF: the grid-wide cell and edge sub-steps of the untiled stacks (UF also forms the layer fluxes on a stack's
 // last sub-step); PH_CS and PH_D: their limiter and their stage's end (tiled stacks end their stage in the tile kernel).
+// PH_P1G / PH_P2G: PH_P1 / PH_P2 with CELL_TRACERS tracers a thread (kernels of their own: they need more registers).
 enum Phase { PH_INIT, PH_LAPE1, PH_LAPCV, PH_LAPE2, PH_A, PH_E, PH_S, PH_ETA, PH_UF, PH_CS, PH_D, PH_POST, PH_P2, PH_P3, PH_P4,
-             PH_P1, PH_P2E, PH_P3E, PH_VMIX, PH_HF1, PH_VHEAT, PH_ONBED };
+             PH_P1, PH_P2E, PH_P3E, PH_VMIX, PH_HF1, PH_VHEAT, PH_ONBED, PH_P1G, PH_P2G };
 
 // Item i of the transport's edge passes: its edge, and its tracers [j0, j1).
 struct EdgeRow {
@@ -186,6 +188,17 @@ __device__ __forceinline__ EdgeRow edge_row(const StackDesc &d, int i) {
   return EdgeRow{j0, min(j0 + d.eg, ntr), i - g * d.M.g.E};
 }
 
+// Item i of the first two cell passes: its cell, its first tracer and how many.
+struct CellRow {
+  int j0, n, c;
+};
+template <int PH>
+__host__ __device__ constexpr int phase_tracers() { return PH == PH_P1G || PH == PH_P2G ? fp64::CELL_TRACERS : 1; }
+__device__ __forceinline__ CellRow cell_row(const StackDesc &d, int i) {
+  const int g = i / d.M.g.N, ntr = d.tr.rows / d.L, j0 = g * d.cg;
+  return CellRow{j0, min(d.cg, ntr - j0), i - g * d.M.g.N};
+}
+
 // Domains of a phase, in block order: which chunk tables its blocks walk.
 template <int PH>
 struct Dom {
@@ -194,7 +207,8 @@ struct Dom {
   static constexpr bool edge = PH == PH_INIT || PH == PH_LAPE1 || PH == PH_LAPE2 || PH == PH_E || PH == PH_S || PH == PH_D ||
                                PH == PH_POST || PH == PH_VMIX || PH == PH_UF;
   static constexpr bool vert = PH == PH_INIT || PH == PH_LAPCV || PH == PH_A;
-  static constexpr bool rows = PH == PH_P1 || PH == PH_P2 || PH == PH_P3 || PH == PH_P4;
+  static constexpr bool rows = PH == PH_P3 || PH == PH_P4;
+  static constexpr bool grows = PH == PH_P1 || PH == PH_P2 || PH == PH_P1G || PH == PH_P2G;
   static constexpr bool erows = PH == PH_POST || PH == PH_P2E || PH == PH_P3E || PH == PH_HF1;
   static constexpr bool wide = PH == PH_ETA || PH == PH_UF;                    // cells / edges in the wide chunks
   static constexpr bool untiled = wide || PH == PH_CS || PH == PH_D;           // of the untiled stacks only
@@ -210,7 +224,7 @@ __host__ __device__ inline int edge_chunks(const Sched &sc) { return Dom<PH>::wi
 template <int PH>
 inline int phase_blocks(const Sched &sc) {
   return (Dom<PH>::cell ? cell_chunks<PH>(sc) : 0) + (Dom<PH>::edge ? edge_chunks<PH>(sc) : 0) + (Dom<PH>::vert ? sc.nvert : 0) +
-         (Dom<PH>::rows ? sc.nrows : 0) + (Dom<PH>::erows ? sc.nerows : 0);
+         (Dom<PH>::rows ? sc.nrows : 0) + (Dom<PH>::grows ? sc.ngrows : 0) + (Dom<PH>::erows ? sc.nerows : 0);
 }
 
 // The chunk of block b of a phase and its kind (0 cell, 1 edge, 2 vertex, 3 (tracer, cell), 4 (tracer, edge)), or -1.
@@ -227,6 +241,7 @@ __device__ __forceinline__ int phase_chunk(const Sched &sc, int b, Chunk &ch) {
     b -= n;
   }
   if (Dom<PH>::vert) { if (b < sc.nvert) { ch = sc.vert[b]; return 2; } b -= sc.nvert; }
+  if (Dom<PH>::grows) { if (b < sc.ngrows) { ch = sc.grows[b]; return 3; } b -= sc.ngrows; }
   if (Dom<PH>::rows) { if (b < sc.nrows) { ch = sc.rows[b]; return 3; } b -= sc.nrows; }
   if (Dom<PH>::erows) { if (b < sc.nerows) { ch = sc.erows[b]; return 4; } }
   return -1;

@@ -104,12 +104,14 @@ __global__ void __launch_bounds__(THREADS) k_phase_m(const StackDesc *__restrict
     ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
     }
   } else if (PH == PH_P1) {
-    ISW_BATCH_L(d.L, LMAXK, mixed::tr_c1<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
+    const CellRow r = cell_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, (mixed::tr_c1<LL, phase_tracers<PH>()>(d.T, d.tr, r.j0, r.n, r.c)));
   } else if (PH == PH_P2E) {
     const EdgeRow r = edge_row(d, i);
     ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 2, r.j0, r.j1, r.e));
   } else if (PH == PH_P2) {
-    ISW_BATCH_L(d.L, LMAXK, mixed::tr_c2<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
+    const CellRow r = cell_row(d, i);
+    ISW_BATCH_L(d.L, LMAXK, (mixed::tr_c2<LL, phase_tracers<PH>()>(d.T, d.tr, r.j0, r.n, r.c)));
   } else if (PH == PH_P3E) {
     const EdgeRow r = edge_row(d, i);
     ISW_BATCH_L(d.L, LMAXK, mixed::tr_a_edge<LL>(d.T, d.tr, r.j0, r.j1, r.e));

@@ -27,70 +27,72 @@ __global__ void __launch_bounds__(THREADS) k_mass(const GridDev g, int L, const 
   M1[(size_t)l * g.N + i] = fp64::mass_cell(g, M0, Fm + (size_t)l * g.E, l, i);
 }
 
-#define ISW_TR_L(LV, CALL)                              \
-  do {                                                  \
-    switch (LV) {                                       \
-      case 1: { constexpr int LL = 1; CALL; } break;    \
-      case 2: { constexpr int LL = 2; CALL; } break;    \
-      case 3: { constexpr int LL = 3; CALL; } break;    \
-      case 4: { constexpr int LL = 4; CALL; } break;    \
-      case 5: { constexpr int LL = 5; CALL; } break;    \
-      case 6: { constexpr int LL = 6; CALL; } break;    \
-      case 7: { constexpr int LL = 7; CALL; } break;    \
-      case 8: { constexpr int LL = 8; CALL; } break;    \
-      default: break;                                   \
-    }                                                   \
+// (the kernels are instances of their layer count, so that a stack of few layers keeps its registers)
+#define ISW_TR_L(LV, ...)                                       \
+  do {                                                          \
+    switch (LV) {                                               \
+      case 1: { constexpr int LL = 1; __VA_ARGS__; } break;     \
+      case 2: { constexpr int LL = 2; __VA_ARGS__; } break;     \
+      case 3: { constexpr int LL = 3; __VA_ARGS__; } break;     \
+      case 4: { constexpr int LL = 4; __VA_ARGS__; } break;     \
+      case 5: { constexpr int LL = 5; __VA_ARGS__; } break;     \
+      case 6: { constexpr int LL = 6; __VA_ARGS__; } break;     \
+      case 7: { constexpr int LL = 7; __VA_ARGS__; } break;     \
+      case 8: { constexpr int LL = 8; __VA_ARGS__; } break;     \
+      default: break;                                           \
+    }                                                           \
   } while (0)
 
 // one thread per (tracer j, cell i), every layer of it
+template <int L>
 __global__ void __launch_bounds__(THREADS) k_p1(const TransportDev T, const TrArgs a, int ntr, int order) {
   pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.g.N * ntr) return;
-  ISW_TR_L(a.L, fp64::tr_p1<LL>(T, a, order, false, t / T.g.N, t % T.g.N));
+  if (t < T.g.N * ntr) fp64::tr_p1<L>(T, a, order, false, t / T.g.N, t % T.g.N);
 }
 
 // one thread per (eg tracers, edge)
+template <int L>
 __global__ void __launch_bounds__(THREADS) k_hf(const TransportDev T, const TrArgs a, int ntr, int eg, int stage) {
   pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, j0 = t / T.g.E * eg;
-  if (j0 >= ntr) return;
-  ISW_TR_L(a.L, fp64::tr_hf_edge<LL>(T, a, stage, j0, min(j0 + eg, ntr), t % T.g.E));
+  if (j0 < ntr) fp64::tr_hf_edge<L>(T, a, stage, j0, min(j0 + eg, ntr), t % T.g.E);
 }
 
+template <int L>
 __global__ void __launch_bounds__(THREADS) k_aflux(const TransportDev T, const TrArgs a, int ntr, int eg) {
   pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, j0 = t / T.g.E * eg;
-  if (j0 >= ntr) return;
-  ISW_TR_L(a.L, fp64::tr_a_edge<LL>(T, a, j0, min(j0 + eg, ntr), t % T.g.E));
+  if (j0 < ntr) fp64::tr_a_edge<L>(T, a, j0, min(j0 + eg, ntr), t % T.g.E);
 }
 
+// one thread per (G tracers, cell)
+template <int L, int G>
 __global__ void __launch_bounds__(THREADS) k_c1(const TransportDev T, const TrArgs a, int ntr) {
   pdl_enter();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.g.N * ntr) return;
-  ISW_TR_L(a.L, fp64::tr_c1<LL>(T, a, t / T.g.N, t % T.g.N, false));
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j0 = t / T.g.N * G;
+  if (j0 < ntr) fp64::tr_c1<L, G>(T, a, j0, min(G, ntr - j0), t % T.g.N, false);
 }
 
+template <int L, int G>
 __global__ void __launch_bounds__(THREADS) k_c2(const TransportDev T, const TrArgs a, int ntr) {
   pdl_enter();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.g.N * ntr) return;
-  ISW_TR_L(a.L, fp64::tr_c2<LL>(T, a, t / T.g.N, t % T.g.N));
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j0 = t / T.g.N * G;
+  if (j0 < ntr) fp64::tr_c2<L, G>(T, a, j0, min(G, ntr - j0), t % T.g.N);
 }
 
+template <int L>
 __global__ void __launch_bounds__(THREADS) k_c3(const TransportDev T, const TrArgs a, int ntr) {
   pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.g.N * ntr) return;
-  ISW_TR_L(a.L, fp64::tr_c3<LL>(T, a, t / T.g.N, t % T.g.N));
+  if (t < T.g.N * ntr) fp64::tr_c3<L>(T, a, t / T.g.N, t % T.g.N);
 }
 
+template <int L>
 __global__ void __launch_bounds__(THREADS) k_p4(const TransportDev T, const TrArgs a, int ntr) {
   pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.g.N * ntr) return;
-  ISW_TR_L(a.L, fp64::tr_p4<LL>(T, a, t / T.g.N, t % T.g.N));
+  if (t < T.g.N * ntr) fp64::tr_p4<L>(T, a, t / T.g.N, t % T.g.N);
 }
 
 // order 1: td out
@@ -206,16 +208,19 @@ int isw_transport_step_many(isw_transport *t, const double *M0, const double *M1
     // the first kernel takes plain stream order, the others are programmatic dependents of the one before (8 tracers of 5
     // layers at level 6: 345 -> 334 us)
     if (order == 1) {
-      launch_kernel(k_p1, nb, st, false, 0, t->d, a, ntr, order);
+      ISW_TR_L(t->L, launch_kernel(k_p1<LL>, nb, st, false, 0, t->d, a, ntr, order));
       launch_kernel(k_td_out, blocks_for((long long)t->d.g.N * a.rows), st, true, 0, t->d, a);
     } else {
-      launch_kernel(k_hf, ne, st, false, 0, t->d, a, ntr, eg, 1);
-      launch_kernel(k_c1, nb, st, true, 0, t->d, a, ntr);
-      launch_kernel(k_hf, ne, st, true, 0, t->d, a, ntr, eg, 2);
-      launch_kernel(k_c2, nb, st, true, 0, t->d, a, ntr);
-      launch_kernel(k_aflux, ne, st, true, 0, t->d, a, ntr, eg);
-      launch_kernel(k_c3, nb, st, true, 0, t->d, a, ntr);
-      launch_kernel(k_p4, nb, st, true, 0, t->d, a, ntr);
+      const int cg = fp64::cell_tracers((long long)t->d.g.N * ntr, t->L);
+      const int ng = blocks_for((long long)t->d.g.N * ((ntr + cg - 1) / cg));
+      constexpr int CG = fp64::CELL_TRACERS;
+      ISW_TR_L(t->L, launch_kernel(k_hf<LL>, ne, st, false, 0, t->d, a, ntr, eg, 1));
+      ISW_TR_L(t->L, launch_kernel(cg == 1 ? k_c1<LL, 1> : k_c1<LL, LL <= 3 ? CG : 1>, ng, st, true, 0, t->d, a, ntr));
+      ISW_TR_L(t->L, launch_kernel(k_hf<LL>, ne, st, true, 0, t->d, a, ntr, eg, 2));
+      ISW_TR_L(t->L, launch_kernel(cg == 1 ? k_c2<LL, 1> : k_c2<LL, LL <= 3 ? CG : 1>, ng, st, true, 0, t->d, a, ntr));
+      ISW_TR_L(t->L, launch_kernel(k_aflux<LL>, ne, st, true, 0, t->d, a, ntr, eg));
+      ISW_TR_L(t->L, launch_kernel(k_c3<LL>, nb, st, true, 0, t->d, a, ntr));
+      ISW_TR_L(t->L, launch_kernel(k_p4<LL>, nb, st, true, 0, t->d, a, ntr));
     }
     ISW_CUDA(cudaGetLastError());
   });

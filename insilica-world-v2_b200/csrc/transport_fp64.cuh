@@ -377,24 +377,33 @@ __device__ __forceinline__ void tr_a_edge(const TransportDev &T, const TrArgs &a
   }
 }
 
+// Tracers of one thread of the first two cell passes (n of them, at most G = CELL_TRACERS): they share the masses, the
+// edges and the fluxes (a third of the pass's loads). Taken in the FP64 form (level-7 member 1.855 -> 1.801 ms) where that leaves CELL_THREADS threads and columns of at most 3
+// layers keep the two tracers' sums in registers (at 5 layers two tracers a thread made 8 tracers' step 299 -> 319 us).
+constexpr int CELL_TRACERS = 2;
+constexpr long long CELL_THREADS = 148 * 960;
+inline int cell_tracers(long long items, int L) { return L <= 3 && items >= CELL_TRACERS * CELL_THREADS ? CELL_TRACERS : 1; }
+
 // cell pass of stage 1: td and p1 from the stage-1 edge fluxes; with_mass: M1 formed here (tracer 0 stores it), else
 // the caller's M1 (Transport.step_many after mass_after)
-template <int L>
-__device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, int j, int i, bool with_mass = true) {
+template <int L, int G>
+__device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, int j0, int n, int i, bool with_mass = true) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
   CellEdges c;
   load_edges(g, i, c);
-  double m1[L], td[L], s[L], mx[L], own[L];
+  double m1[L], mx[L], td[G][L], s[G][L], own[G][L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
-    const double m0 = a.M0[om], pi = a.tr[j][om];
-    own[l] = pi;
+    const double m0 = a.M0[om];
     m1[l] = m0;
-    td[l] = m0 * pi;
-    s[l] = m0 * pi;
     mx[l] = m0;
+#pragma unroll
+    for (int t = 0; t < G; t++) {
+      own[t][l] = t < n ? a.tr[j0 + t][om] : 0.0;
+      td[t][l] = s[t][l] = m0 * own[t][l];
+    }
   }
   const double frac = 1.0 / 3.0;
 #pragma unroll
@@ -402,48 +411,64 @@ __device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, in
     const int e = c.e[q];
     if (e >= 0) {
       const bool out = c.out[q];
-      double Av[L];
-      ld_layers<L>(T.A + fx(j, E, e, L), Av);
+      double f[L];
 #pragma unroll
       for (int l = 0; l < L; l++) {
-        const double *p = a.tr[j] + (size_t)l * N;
-        const double f = a.Fm[(size_t)l * E + e];
-        const double pn = p[c.nb[q]];
-        const double fu = upwind_v(f, out ? own[l] : pn, out ? pn : own[l]);
-        const double hf = frac * Av[l];
-        const double m = frac * f;
-        if (out) { m1[l] -= f; td[l] -= fu; s[l] -= hf; mx[l] -= m; }
-        else { m1[l] += f; td[l] += fu; s[l] += hf; mx[l] += m; }
+        f[l] = a.Fm[(size_t)l * E + e];
+        const double m = frac * f[l];
+        if (out) { m1[l] -= f[l]; mx[l] -= m; }
+        else { m1[l] += f[l]; mx[l] += m; }
       }
+#pragma unroll
+      for (int t = 0; t < G; t++)
+        if (t < n) {
+          double Av[L];
+          ld_layers<L>(T.A + fx(j0 + t, E, e, L), Av);
+#pragma unroll
+          for (int l = 0; l < L; l++) {
+            const double pn = a.tr[j0 + t][(size_t)l * N + c.nb[q]];
+            const double fu = upwind_v(f[l], out ? own[t][l] : pn, out ? pn : own[t][l]);
+            const double hf = frac * Av[l];
+            if (out) { td[t][l] -= fu; s[t][l] -= hf; }
+            else { td[t][l] += fu; s[t][l] += hf; }
+          }
+        }
     }
   }
-  double tdo[L], p1o[L];
 #pragma unroll
-  for (int l = 0; l < L; l++) {
-    const size_t om = (size_t)l * N + i;
-    double mm = m1[l];
-    if (with_mass) { if (j == 0) a.M1[om] = mm; }
-    else mm = a.M1[om];
-    tdo[l] = td[l] / mm;
-    p1o[l] = s[l] / mx[l];
+  for (int t = 0; t < G; t++) {
+    if (t >= n) break;
+    const int j = j0 + t;
+    double tdo[L];
+    double p1o[L];
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+      const size_t om = (size_t)l * N + i;
+      double mm = m1[l];
+      if (with_mass) { if (j == 0) a.M1[om] = mm; }
+      else mm = a.M1[om];
+      tdo[l] = td[t][l] / mm;
+      p1o[l] = (s[t][l] / mx[l]);
+    }
+    st_layers<L>(T.td + fx(j, N, i, L), tdo);
+    st_layers<L>(T.p1 + fx(j, N, i, L), p1o);
   }
-  st_layers<L>(T.td + fx(j, N, i, L), tdo);
-  st_layers<L>(T.p1 + fx(j, N, i, L), p1o);
 }
 
 // cell pass of stage 2: p2 from the stage-2 edge fluxes
-template <int L>
-__device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, int j, int i) {
+template <int L, int G>
+__device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, int j0, int n, int i) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
   CellEdges c;
   load_edges<false>(g, i, c);
-  double s[L], mx[L];
+  double mx[L], s[G][L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
-    s[l] = a.M0[om] * a.tr[j][om];
     mx[l] = a.M0[om];
+#pragma unroll
+    for (int t = 0; t < G; t++) s[t][l] = t < n ? mx[l] * a.tr[j0 + t][om] : 0.0;
   }
   const double frac = 1.0 / 2.0;
 #pragma unroll
@@ -451,21 +476,32 @@ __device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, in
     const int e = c.e[q];
     if (e >= 0) {
       const bool out = c.out[q];
-      double Av[L];
-      ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll
       for (int l = 0; l < L; l++) {
-        const double f = a.Fm[(size_t)l * E + e];
-        const double hf = frac * Av[l];
-        const double m = frac * f;
-        if (out) { s[l] -= hf; mx[l] -= m; } else { s[l] += hf; mx[l] += m; }
+        const double m = frac * a.Fm[(size_t)l * E + e];
+        if (out) mx[l] -= m; else mx[l] += m;
       }
+#pragma unroll
+      for (int t = 0; t < G; t++)
+        if (t < n) {
+          double Av[L];
+          ld_layers<L>(T.A + fx(j0 + t, E, e, L), Av);
+#pragma unroll
+          for (int l = 0; l < L; l++) {
+            const double hf = frac * Av[l];
+            if (out) s[t][l] -= hf; else s[t][l] += hf;
+          }
+        }
     }
   }
-  double p2o[L];
 #pragma unroll
-  for (int l = 0; l < L; l++) p2o[l] = s[l] / mx[l];
-  st_layers<L>(T.p2 + fx(j, N, i, L), p2o);
+  for (int t = 0; t < G; t++) {
+    if (t >= n) break;
+    double p2o[L];
+#pragma unroll
+    for (int l = 0; l < L; l++) p2o[l] = (s[t][l] / mx[l]);
+    st_layers<L>(T.p2 + fx(j0 + t, N, i, L), p2o);
+  }
 }
 
 // cell pass of stage 3: the Zalesak ratios from the antidiffusive fluxes and the bounds of psi and td

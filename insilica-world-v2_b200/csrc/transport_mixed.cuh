@@ -156,22 +156,24 @@ __device__ __forceinline__ void tr_a_edge(const TransportDev &T, const TrArgs &a
   }
 }
 
-template <int L>
-__device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, int j, int i) {
+template <int L, int G>
+__device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, int j0, int n, int i) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
   fp64::CellEdges c;
   fp64::load_edges(g, i, c);
-  double m1[L], td[L], s[L], mx[L], own[L];
+  double m1[L], mx[L], td[G][L], s[G][L], own[G][L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
-    const double m0 = a.M0[om], pi = a.tr[j][om];
-    own[l] = pi;
+    const double m0 = a.M0[om];
     m1[l] = m0;
-    td[l] = m0 * pi;
-    s[l] = m0 * pi;
     mx[l] = m0;
+#pragma unroll
+    for (int t = 0; t < G; t++) {
+      own[t][l] = t < n ? a.tr[j0 + t][om] : 0.0;
+      td[t][l] = s[t][l] = m0 * own[t][l];
+    }
   }
   const double frac = 1.0 / 3.0;
 #pragma unroll
@@ -179,46 +181,62 @@ __device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, in
     const int e = c.e[q];
     if (e >= 0) {
       const bool out = c.out[q];
-      double Av[L];
-      ld_layers<L>(T.A + fx(j, E, e, L), Av);
+      double f[L];
 #pragma unroll
       for (int l = 0; l < L; l++) {
-        const double *p = a.tr[j] + (size_t)l * N;
-        const double f = a.Fm[(size_t)l * E + e];
-        const double pn = p[c.nb[q]];
-        const double fu = fp64::upwind_v(f, out ? own[l] : pn, out ? pn : own[l]);
-        const double hf = frac * Av[l];
-        const double m = frac * f;
-        if (out) { m1[l] -= f; td[l] -= fu; s[l] -= hf; mx[l] -= m; }
-        else { m1[l] += f; td[l] += fu; s[l] += hf; mx[l] += m; }
+        f[l] = a.Fm[(size_t)l * E + e];
+        const double m = frac * f[l];
+        if (out) { m1[l] -= f[l]; mx[l] -= m; }
+        else { m1[l] += f[l]; mx[l] += m; }
       }
+#pragma unroll
+      for (int t = 0; t < G; t++)
+        if (t < n) {
+          double Av[L];
+          ld_layers<L>(T.A + fx(j0 + t, E, e, L), Av);
+#pragma unroll
+          for (int l = 0; l < L; l++) {
+            const double pn = a.tr[j0 + t][(size_t)l * N + c.nb[q]];
+            const double fu = fp64::upwind_v(f[l], out ? own[t][l] : pn, out ? pn : own[t][l]);
+            const double hf = frac * Av[l];
+            if (out) { td[t][l] -= fu; s[t][l] -= hf; }
+            else { td[t][l] += fu; s[t][l] += hf; }
+          }
+        }
     }
   }
-  double tdo[L];
-  float p1o[L];
 #pragma unroll
-  for (int l = 0; l < L; l++) {
-    const size_t om = (size_t)l * N + i;
-    if (j == 0) a.M1[om] = m1[l];
-    tdo[l] = td[l] / m1[l];
-    p1o[l] = (float)(s[l] / mx[l]);
+  for (int t = 0; t < G; t++) {
+    if (t >= n) break;
+    const int j = j0 + t;
+    double tdo[L];
+    float p1o[L];
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+      const size_t om = (size_t)l * N + i;
+      const double mm = m1[l];
+      if (j == 0) a.M1[om] = mm;
+      tdo[l] = td[t][l] / mm;
+      p1o[l] = (float)(s[t][l] / mx[l]);
+    }
+    st_layers<L>(T.td + fx(j, N, i, L), tdo);
+    st_layers<L>(T.p1f + fx(j, N, i, L), p1o);
   }
-  st_layers<L>(T.td + fx(j, N, i, L), tdo);
-  st_layers<L>(T.p1f + fx(j, N, i, L), p1o);
 }
 
-template <int L>
-__device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, int j, int i) {
+template <int L, int G>
+__device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, int j0, int n, int i) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
   fp64::CellEdges c;
   fp64::load_edges<false>(g, i, c);
-  double s[L], mx[L];
+  double mx[L], s[G][L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
-    s[l] = a.M0[om] * a.tr[j][om];
     mx[l] = a.M0[om];
+#pragma unroll
+    for (int t = 0; t < G; t++) s[t][l] = t < n ? mx[l] * a.tr[j0 + t][om] : 0.0;
   }
   const double frac = 1.0 / 2.0;
 #pragma unroll
@@ -226,21 +244,32 @@ __device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, in
     const int e = c.e[q];
     if (e >= 0) {
       const bool out = c.out[q];
-      double Av[L];
-      ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll
       for (int l = 0; l < L; l++) {
-        const double f = a.Fm[(size_t)l * E + e];
-        const double hf = frac * Av[l];
-        const double m = frac * f;
-        if (out) { s[l] -= hf; mx[l] -= m; } else { s[l] += hf; mx[l] += m; }
+        const double m = frac * a.Fm[(size_t)l * E + e];
+        if (out) mx[l] -= m; else mx[l] += m;
       }
+#pragma unroll
+      for (int t = 0; t < G; t++)
+        if (t < n) {
+          double Av[L];
+          ld_layers<L>(T.A + fx(j0 + t, E, e, L), Av);
+#pragma unroll
+          for (int l = 0; l < L; l++) {
+            const double hf = frac * Av[l];
+            if (out) s[t][l] -= hf; else s[t][l] += hf;
+          }
+        }
     }
   }
-  float p2o[L];
 #pragma unroll
-  for (int l = 0; l < L; l++) p2o[l] = (float)(s[l] / mx[l]);
-  st_layers<L>(T.p2f + fx(j, N, i, L), p2o);
+  for (int t = 0; t < G; t++) {
+    if (t >= n) break;
+    float p2o[L];
+#pragma unroll
+    for (int l = 0; l < L; l++) p2o[l] = (float)(s[t][l] / mx[l]);
+    st_layers<L>(T.p2f + fx(j0 + t, N, i, L), p2o);
+  }
 }
 
 template <int L>

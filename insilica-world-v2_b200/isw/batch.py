@@ -187,7 +187,7 @@ class Batch:
         _lib.check(_lib.isw_batch_flush(self._h, stream_of(self.device, stream)))
 
     def status(self, reset=False, stream=None):
-        """The device status word: 0, ISW_ETIMEOUT (5) after a grid barrier's bounded wait ran out, or ISW_ENOTFINITE (6)
+        """The device status word: 0, ISW_ETIMEOUT (5) after a tile's (or the grid barrier's) bounded wait ran out, or ISW_ENOTFINITE (6)
         after a step left a NaN or Inf thickness. While it is set, step() raises IswError with that status; reset clears
         it (restore the state first)."""
         st = _lib.isw_batch_status(self._h, stream_of(self.device, stream), 1 if reset else 0)
