@@ -17,6 +17,11 @@
 // buffers suffice: a tile publishes round r + 2 only after its neighbours raised round r + 1, which they do after reading
 // round r.
 //
+// What bounds it: a sub-step is 1.9 us FP64 (1.1 mixed) on tiles of 553 cells, of whose 3,600 cycles some 2,300 move
+// shared-memory wavefronts (a third of them bank conflicts of the gathers); an exchange 3 us, staging 7, the stage's end 15.
+// Before (constants in shared memory, a grid barrier an exchange, C and D as launches of their own) a level-6 member took
+// 0.589 ms FP64 and 0.447 mixed, with this kernel 0.497 and 0.371 (nothing else changed).
+//
 // The FP64 form's values are the grid-wide passes' bit for bit: a cell sums +-(l_e H_e ub), rounded once per edge, in its
 // slot order (rounding is symmetric in sign, and a sum that started from +0 is unchanged by the padded slot's zero); the
 // limiter sums in ascending edge order. Compiled with
