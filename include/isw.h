@@ -164,8 +164,11 @@ int isw_layers_vmix_heat(isw_layers *s, const double *h, const double *diss, dou
 /* Zero the wall edges (wall[e] == 0) of the first `rows` rows (1..8) of an edge field a (rows x E); no-op without walls. */
 int isw_layers_mask(isw_layers *s, double *a, int rows, void *stream);
 /* The status word of the one-stack batch that isw_layers_step uses (as isw_batch_status; ISW_OK when the handle steps
- * call by call). While it holds ISW_ETIMEOUT or ISW_ENOTFINITE, isw_layers_step refuses with that status. */
+ * call by call). While it holds ISW_ETIMEOUT, isw_layers_step refuses with that status, and while it holds ISW_ENOTFINITE
+ * too, unless the stack has option branches. */
 int isw_layers_status(isw_layers *s, void *stream, int reset);
+/* Failure-detection test of that batch (isw_batch_fault_test); ISW_EUNSUPPORTED before the first step through it. */
+int isw_layers_fault_test(isw_layers *s, long long timeout_ns, void *stream);
 /* Replace the bottom height b (N values, a DEVICE pointer, copied on `stream`) the layers rest on: the reference's
  * Layers.b (layers.py:55), which it fixes at construction; here a served request's layers are reused for the next
  * request of the same kind with that request's own terrain. */

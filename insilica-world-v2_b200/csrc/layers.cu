@@ -506,6 +506,9 @@ void layers_step(isw_layers *s, double *h, double *u, double *Fm, double *theta,
     layers_step_solo(s, h, u, Fm, dt, nfast, true, st);
     return;
   }
+  if (s->solo && isw_batch_pending(s->solo) == ISW_ETIMEOUT)   // whichever way this call would go
+    fail(ISW_ETIMEOUT, "layers.step: refused: an earlier step's wait on the device timed out, so the state is half-updated; "
+                       "restore it and clear the status (isw_layers_status with reset) to step again");
   const LayersDev &D = s->d;
   if (!s->percall && !D.air) {
     const bool options = D.wall || D.ob || D.shelf > 0 || D.sig || D.tide || D.cbot || D.cd_bot > 0;
@@ -516,7 +519,8 @@ void layers_step(isw_layers *s, double *h, double *u, double *Fm, double *theta,
     if (options) {
       // option stacks: the private batch once a call repeats the one before it with no option set in between. Building it
       // costs more than recording the per-call graph, of which eight are kept, so alternating arrays and options set before
-      // every step stay with the graphs. Never under a capture, nor while that batch would refuse to step.
+      // every step stay with the graphs. Never under a capture, nor while that batch would refuse to step for a non-finite
+      // thickness that a step without options left: option stacks are stepped whatever their thicknesses.
       solo = cs0 == cudaStreamCaptureStatusNone && s->last_version == s->version && same_call(s->last_key, h, u, Fm, dt, nfast) &&
              !(s->solo && isw_batch_pending(s->solo));
       s->last_key = GraphEntry{h, u, Fm, nullptr, dt, nfast, nullptr};
@@ -758,6 +762,15 @@ int isw_layers_status(isw_layers *s, void *stream, int reset) {
   }
   if (!s->solo) return ISW_OK;                  // only the batched one-stack path keeps a status word
   return isw_batch_status(s->solo, stream, reset);
+}
+
+int isw_layers_fault_test(isw_layers *s, long long timeout_ns, void *stream) {
+  return guarded([&] {
+    if (!s) fail(ISW_EINVAL, "layers.fault_test: null handle");
+    if (!s->solo) fail(ISW_EUNSUPPORTED, "layers.fault_test: the handle has not stepped through its private batch");
+    const int rc = isw_batch_fault_test(s->solo, timeout_ns, stream);
+    if (rc != ISW_OK) fail(rc, isw_last_error());
+  });
 }
 
 int isw_layers_lap(isw_layers *s, const double *u, double *out, void *stream) {

@@ -158,13 +158,17 @@ class Layers:
         self.b.copy_(bt)
 
     def status(self, reset=False, stream=None):
-        """The status word of the one-stack batch this Layers steps through: 0, ISW_ETIMEOUT (5) after a fast-loop barrier
-        timed out, or ISW_ENOTFINITE (6) after a step left a NaN or Inf thickness. While it is set, step() raises; reset
-        clears it (restore the state first)."""
+        """The status word of the one-stack batch this Layers steps through: 0, ISW_ETIMEOUT (5) after a wait of the fast
+        loop ran out, or ISW_ENOTFINITE (6) after a step left a NaN or Inf thickness. While it is set, step() raises (a
+        stack with option branches only for ISW_ETIMEOUT); reset clears it (restore the state first)."""
         st = _lib.isw_layers_status(self._h, stream_of(self.dg.device, stream), 1 if reset else 0)
         if st not in (_lib.ISW_OK, _lib.ISW_ETIMEOUT, _lib.ISW_ENOTFINITE):
             _lib.check(st)
         return st
+
+    def fault_test(self, timeout_s=0.05, stream=None):
+        """Batch.fault_test on the one-stack batch this Layers steps through (it must have stepped through it before)."""
+        _lib.check(_lib.isw_layers_fault_test(self._h, int(timeout_s * 1e9), stream_of(self.dg.device, stream)))
 
     def step(self, h, u, dt, nfast, Fm=None, theta=None, stream=None):
         """One time-split RK3 step in place on h (L, N), u (L, E), with nfast fast sub-steps per full step (stage s takes

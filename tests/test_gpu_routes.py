@@ -61,3 +61,54 @@ def test_option_routes_equal_per_call(grid4, options):
     torch.cuda.synchronize()
     assert all(core.status() == 0 for core in cores)
     assert torch.equal(*(torch.nan_to_num(ss[0]['h'], nan=-1.0) for ss in sets))
+
+
+def test_timed_out_option_stack_is_refused(grid4):
+    """A wait of the tile kernel that runs out on an option stack: every later step is refused with ISW_ETIMEOUT (a call
+    that repeats the one before it, one with other arguments, one after an option was set, one inside a capture), and
+    after a reset the stack steps on equal to the call-by-call kernels bit for bit (the launch that timed out wrote
+    scratch only)."""
+    from isw._lib import ISW_ETIMEOUT, IswError
+    from isw.gpu import DeviceGrid
+    from isw.layers import Layers
+    z = golden('options_n4')
+    dg = DeviceGrid(grid4)
+    dt, nfast = float(z['dt']), int(z['nfast'])
+    cores, states = [], []
+    for batched in (True, False):
+        cores.append(Layers(dg, 2, b=z['b'], gprime=[0.02], floor=1.0, batched=batched, wall=z['wall']))
+        states.append((T(z['h0']), T(z['u0']) * T(z['wall']), torch.zeros_like(T(z['u0']))))
+
+    def step(which, n=nfast):
+        h, u, Fm = states[which]
+        cores[which].step(h, u, dt, n, Fm)
+    for _ in range(2):                                  # the second goes through the private batch
+        step(0)
+        step(1)
+    core = cores[0]
+    core.fault_test(timeout_s=0.05)
+    torch.cuda.synchronize()
+    assert core.status() == ISW_ETIMEOUT
+
+    def refused(n=nfast):
+        with pytest.raises(IswError) as err:
+            step(0, n)
+        assert err.value.status == ISW_ETIMEOUT
+    refused()
+    refused(nfast + 1)
+    core.cd_bot = 2.5e-3
+    refused()
+    core.cd_bot = 0.0
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            refused()
+    torch.cuda.synchronize()
+    assert core.status(reset=True) == ISW_ETIMEOUT and core.status() == 0
+    for _ in range(3):
+        step(0)
+        step(1)
+    torch.cuda.synchronize()
+    for x, y in zip(*states):
+        assert torch.equal(x, y)
