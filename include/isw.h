@@ -245,7 +245,7 @@ int isw_batch_info(isw_batch *b, int *stacks, int *tiles, int *tile_k, long long
  * after a step left a NaN or Inf thickness (checked for every cell and layer at the end of each step). The kernel that
  * records a failure also writes it to a mapped host word, and isw_batch_step refuses to run (returning that status)
  * until the word is cleared, so later steps never run on a half-updated state. Synchronises `stream`; reset != 0
- * clears the word (restore the state first). */
+ * waits for the device and clears the word (restore the state first); steps in flight on other streams are unharmed. */
 int isw_batch_status(isw_batch *b, void *stream, int reset);
 /* Failure-detection test: the first stage's tile launch with a tile that never raises its flag, so its neighbours'
  * bounded wait runs out after timeout_ns (1 ms .. 2 s) and the status word becomes ISW_ETIMEOUT. Test use only. */

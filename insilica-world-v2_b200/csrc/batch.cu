@@ -1420,11 +1420,12 @@ int isw_batch_status(isw_batch *b, void *stream, int reset) {
     if (!b) fail(ISW_EINVAL, "batch.status: null handle");
     ISW_CUDA(cudaSetDevice(b->device));
     int st = 0;
+    if (reset) ISW_CUDA(cudaDeviceSynchronize());   // steps in flight on any stream: they raise flags and may yet fail
     ISW_CUDA(cudaMemcpyAsync(&st, &b->status->code, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     ISW_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    if (reset) {
+    if (reset && st != ISW_OK) {             // (nothing to clear otherwise; the batch refuses to step until it is cleared)
       ISW_CUDA(cudaMemset(&b->status->code, 0, sizeof(int)));
-      if (b->flags)                          // a launch that timed out left its tiles' flags apart
+      if (st == ISW_ETIMEOUT && b->flags)    // a launch that timed out left its tiles' flags apart
         ISW_CUDA(cudaMemset(b->flags, 0, sizeof(unsigned) * TILE_FLAG_STRIDE * (size_t)b->ntiles));
       ISW_CUDA(cudaDeviceSynchronize());
       *(volatile int *)b->status_host = 0;

@@ -185,6 +185,43 @@ def test_barrier_timeout_refuses_then_recovers(dev, grid4):
         assert torch.equal(x, y)
 
 
+def test_status_reset_beside_steps_in_flight(dev, grid4):
+    """Status resets from one thread while another steps the batch on a stream of its own: the tiles' exchange flags are
+    left alone, no wait runs out, and the state equals an undisturbed run's bit for bit."""
+    import threading
+    from isw.batch import Batch
+    from isw.gpu import DeviceGrid
+    from isw.workload import Member, planet_grid
+    dg = DeviceGrid(planet_grid(grid4))
+    one, two = Batch(0), Batch(0)
+    a, b = Member(dg, 4, nfast=20, batch=one), Member(dg, 4, nfast=20, batch=two)
+    one.step()
+    two.step()
+    assert one.info()['tiles'] > 0
+    torch.cuda.synchronize()
+    done, codes = threading.Event(), []
+
+    def resets():
+        while not done.is_set():
+            codes.append(one.status(reset=True))
+    t = threading.Thread(target=resets)
+    t.start()
+    side = torch.cuda.Stream()
+    try:
+        for _ in range(200):
+            one.step(side)
+    finally:
+        side.synchronize()
+        done.set()
+        t.join()
+    for _ in range(200):
+        two.step()
+    torch.cuda.synchronize()
+    assert codes and set(codes) == {0} and one.status() == 0
+    for x, y in zip(a.state(), b.state()):
+        assert torch.equal(x, y)
+
+
 @pytest.mark.parametrize('precision', ['double', 'mixed'])
 def test_nonfinite_thickness_reported_and_refused(dev, grid4, precision):
     """A NaN written into one thickness from the host: the step that meets it records ISW_ENOTFINITE (checked for every
