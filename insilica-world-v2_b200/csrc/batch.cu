@@ -445,6 +445,22 @@ const TileSetDev &tiles_on_device(isw_grid *g, TileCache *c) {
   return t;
 }
 
+// Layers the stage's end takes at once at interval k: every layer where each tile's share fits a block, else an even split
+// into as few groups as fit (0: not even one layer does).
+int end_group(const TileSetHost &h, int k, int L, bool mixed, int bps) {
+  const size_t budget = bps == 2 ? SMEM_TWO : SMEM_ONE;
+  for (int n = 1; n <= L; n++) {
+    const int lg = (L + n - 1) / n;
+    bool ok = true;
+    for (int p = 0; p < h.P && ok; p++) {
+      const int32_t *nc = &h.ncnt[(size_t)p * (h.k + 1)], *ne = &h.ecnt[(size_t)p * (h.k + 1)];
+      ok = tile_smem_bytes(nc[k], ne[k], nc[1], ne[0], lg, n > 1, mixed) <= budget;
+    }
+    if (ok) return lg;
+  }
+  return 0;
+}
+
 // The smallest kernel capacity whose registers hold every tile of a tiling at interval k (-1: none).
 int tiles_cap(const TileSetHost &h, int k, int bps) {
   const int nt = fast_tiles_threads(bps);
@@ -460,26 +476,25 @@ int tiles_cap(const TileSetHost &h, int k, int bps) {
 }
 
 // The largest k' <= the probe's k at which every tile fits a block: its cells, edges and own cells' edges the
-// threads' registers, what its threads share `budget` bytes of shared memory (0 if none).
+// threads' registers, what its threads share the block's shared memory (0 if none). An interval at which the stage's end
+// takes every layer at once comes before a longer one at which it does not.
 int fitting_k(const TileSetHost &h, int L, bool mixed, int bps) {
-  const size_t budget = bps == 2 ? SMEM_TWO : SMEM_ONE;
+  int grouped = 0;
   for (int kk = h.k; kk >= 1; kk--) {
-    bool ok = tiles_cap(h, kk, bps) >= 0;
-    for (int p = 0; p < h.P && ok; p++) {
-      const int32_t *nc = &h.ncnt[(size_t)p * (h.k + 1)], *ne = &h.ecnt[(size_t)p * (h.k + 1)];
-      ok = tile_smem_bytes(nc[kk], ne[kk], nc[1], ne[0], L, mixed) <= budget;
-    }
-    if (ok) return kk;
+    if (tiles_cap(h, kk, bps) < 0) continue;
+    const int lg = end_group(h, kk, L, mixed, bps);
+    if (lg == L) return kk;
+    if (lg > 0 && grouped == 0) grouped = kk;
   }
-  return 0;
+  return grouped;
 }
 
-// Dynamic shared memory of the largest tile of a tile set.
-size_t tiles_smem(const TileSetHost &h, int L, bool mixed) {
+// Dynamic shared memory of the largest tile of a tile set whose stage's end takes lg of L layers at once.
+size_t tiles_smem(const TileSetHost &h, int lg, int L, bool mixed) {
   size_t worst = 0;
   for (int p = 0; p < h.P; p++) {
     const int32_t *nc = &h.ncnt[(size_t)p * (h.k + 1)], *ne = &h.ecnt[(size_t)p * (h.k + 1)];
-    worst = std::max(worst, tile_smem_bytes(h.cell_off[p + 1] - h.cell_off[p], h.edge_off[p + 1] - h.edge_off[p], nc[1], ne[0], L, mixed));
+    worst = std::max(worst, tile_smem_bytes(h.cell_off[p + 1] - h.cell_off[p], h.edge_off[p + 1] - h.edge_off[p], nc[1], ne[0], lg, lg < L, mixed));
   }
   return worst;
 }
@@ -495,6 +510,7 @@ int kernel_lmax(int L) { return L <= 2 ? 2 : L <= 3 ? 3 : L <= 5 ? 5 : 8; }
 // Stacks whose tiles would not fit in shared memory at all take the grid-wide sub-step kernels.
 struct Tiling {
   int k = 0, bps = 2;                          // k: the smallest exchange interval over the stacks
+  bool grouped = false;                        // a stack's end takes its layers in groups
   double us = 0;                               // modelled time of the step's tile launches
   std::vector<int> P;                          // tiles per slot (0: untiled)
   std::vector<int> K;                          // exchange interval per slot
@@ -521,15 +537,16 @@ bool tiles_form(const isw_batch *b, const BatchSlot &sl) {
 // (staging, the stage's end), per exchange its latency, per sub-step the edges the largest tile updates. The constants are
 // B200 timings of the kernel's phases at levels 6 and 7 (148 tiles of 553 and 1107 cells): staging and end 22 us, an
 // exchange 3.5 us, a sub-step 0.76 ns (FP64) or 0.40 ns (mixed) per edge and tile on the SM and at least 0.7 us.
-double tiles_us(const TileSetHost &h, int k, int nfast, bool mixed, int bps) {
+double tiles_us(const TileSetHost &h, int k, int L, int nfast, bool mixed, int bps) {
   const double cs[3] = {1.0 / 3.0, 1.0 / 2.0, 1.0};
+  const int lg = end_group(h, k, L, mixed, bps);
   std::vector<int> edges(k + 1, 0);            // most edges of ring <= r in a tile
   for (int p = 0; p < h.P; p++)
     for (int r = 0; r <= k; r++) edges[r] = std::max(edges[r], (int)h.ecnt[(size_t)p * (h.k + 1) + r]);
   double us = 0;
   for (double c : cs) {
     const int n = std::max(1, (int)std::ceil(c * nfast));
-    us += 22.0;
+    us += 22.0 + 3.5 * ((L + lg - 1) / lg - 1);
     for (int done = 0; done < n; done += k) {
       const int K = std::min(k, n - done);
       us += 3.5;
@@ -541,18 +558,19 @@ double tiles_us(const TileSetHost &h, int k, int nfast, bool mixed, int bps) {
 
 // The exchange interval of a stack's tiling: the largest that fits when the layout was asked for, else the fastest by
 // the model.
-int pick_k(isw_batch *b, const BatchSlot &sl, int P, int kcap, int bps, double *us) {
+int pick_k(isw_batch *b, const BatchSlot &sl, int P, int kcap, int bps, double *us, bool *grouped) {
   const bool mixed = form_of(sl) == 1;
   int k = fitting_k_or_none(sl.layers->grid, sl.layers->d.L, mixed, P, kcap, bps);
   if (k == 0) return 0;
   const std::shared_ptr<TileCache> set = tiles_for(sl.layers->grid, P, std::min(K_PROBE, kcap));
   const TileSetHost &h = set->host;
-  *us = tiles_us(h, k, sl.nfast, mixed, bps);
+  *us = tiles_us(h, k, sl.layers->d.L, sl.nfast, mixed, bps);
   if (b->layout == 0)
     for (int kk = k - 1; kk >= 1; kk--) {
-      const double t = tiles_us(h, kk, sl.nfast, mixed, bps);
+      const double t = tiles_us(h, kk, sl.layers->d.L, sl.nfast, mixed, bps);
       if (t < *us) { *us = t; k = kk; }
     }
+  if (end_group(h, k, sl.layers->d.L, mixed, bps) < sl.layers->d.L) *grouped = true;
   return k;
 }
 
@@ -576,7 +594,7 @@ Tiling plan_shared(isw_batch *b, int bps) {
     const int Pq = std::max(1, (int)((long long)slots * N / std::max(1LL, cells_total[form_of(sl)])));
     if (Pq * 16 > N) return Tiling{};          // tiles of at least 16 owned cells, for every stack
     double us = 0;
-    const int kf = pick_k(b, sl, Pq, b->tile_k, bps, &us);
+    const int kf = pick_k(b, sl, Pq, b->tile_k, bps, &us, &t.grouped);
     if (kf == 0) return Tiling{};
     t.P[q] = Pq;
     t.K[q] = kf;
@@ -611,7 +629,7 @@ Tiling plan_packed(isw_batch *b, int bps) {
     const int N = sl.layers->grid->d.N;
     const int Pq = std::min(cap, std::max(1, (N + cells - 1) / cells));
     if (Pq * 16 > N) continue;
-    const int kf = pick_k(b, sl, Pq, kcap, bps, &slot_us[q]);
+    const int kf = pick_k(b, sl, Pq, kcap, bps, &slot_us[q], &t.grouped);
     if (kf == 0) continue;
     t.P[q] = Pq;
     t.K[q] = kf;                               // each stack its own interval: a group's rounds follow its slowest
@@ -645,12 +663,13 @@ bool resident(isw_batch *b, const Tiling &t) {
     for (size_t q = 0; q < b->slots.size(); q++)
       if (t.P[q] > 0 && form_of(b->slots[q]) == f) {
         count[t.group[q]] += t.P[q];
-        smax = std::max(smax, tiles_smem(tiles_for(b->slots[q].layers->grid, t.P[q], t.K[q])->host, b->slots[q].layers->d.L, f == 1));
+        const std::shared_ptr<TileCache> set = tiles_for(b->slots[q].layers->grid, t.P[q], t.K[q]);
+        const int L = b->slots[q].layers->d.L;
+        smax = std::max(smax, tiles_smem(set->host, end_group(set->host, t.K[q], L, f == 1, t.bps), L, f == 1));
       }
     if (count.empty()) continue;
-    for (int kind = 0; kind < 4; kind++) {
-      if (f == 1 && kind >= 2) break;          // (walls are the FP64 form's)
-      const void *fn = fast_tiles_kernel(t.bps, kind & 1, kind >= 2 ? 2 : f);
+    for (int kind = 0; kind < (f == 1 ? 3 : 6); kind++) {      // capacities, then (FP64) with walls
+      const void *fn = fast_tiles_kernel(t.bps, kind % 3, kind >= 3 ? 2 : f);
       // the kernel's limit is one setting for every batch: always the most a tile may ask for
       ISW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(t.bps == 2 ? SMEM_TWO : SMEM_ONE)));
       int per = 0;
@@ -689,7 +708,8 @@ void rebuild(isw_batch *b) {
       for (int lay = 1; lay <= 2; lay++) {
         if (b->layout != 0 && b->layout != lay) continue;
         Tiling t = lay == 1 ? plan_shared(b, bps) : plan_packed(b, bps);
-        if (t.k > 0 && (best.k == 0 || t.us < best.us)) best = t;
+        // (layers in groups only where no layout takes them together)
+        if (t.k > 0 && (best.k == 0 || t.grouped < best.grouped || (t.grouped == best.grouped && t.us < best.us))) best = t;
       }
     }
   }
@@ -742,10 +762,11 @@ void rebuild(isw_batch *b) {
       const int g = best.group[q];
       d.tiled = 1;
       d.tiles = tiles_on_device(sl.layers->grid, tc.get());
-      gsmem[g] = std::max(gsmem[g], tiles_smem(tc->host, d.L, form_of(sl) == 1));
+      d.lg = end_group(tc->host, best.K[q], d.L, form_of(sl) == 1, best.bps);
+      gsmem[g] = std::max(gsmem[g], tiles_smem(tc->host, d.lg, d.L, form_of(sl) == 1));
       gform[g] = form_of(sl);
       if (d.M.wall) gwalls[g] = 1;
-      gcap[g] = std::max(gcap[g], tiles_cap(tc->host, best.K[q], best.bps));
+      gcap[g] = std::max(gcap[g], d.lg < d.L ? 2 : tiles_cap(tc->host, best.K[q], best.bps));
       gfirst.emplace_back((size_t)g, (int)grefs[g].size());
       for (int p = 0; p < best.P[q]; p++) grefs[g].push_back(TileRef{s, p});
     }

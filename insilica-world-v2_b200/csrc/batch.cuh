@@ -37,6 +37,7 @@ struct StackDesc {
   int n[3];
   double cdt[3], tau[3], inv_n[3];
   TileSetDev tiles;
+  int lg;                    // tiled: layers whose fluxes the stage's end holds at once
   int tile_base;             // the stack's first tile in the batch's list (and its first flag)
 };
 

@@ -85,6 +85,152 @@ __device__ __forceinline__ float slot_flux(const float *fl, unsigned v) { return
 // Bit 15 of an edge's local cells: a thin wall closes it (tiles have at most 32000 cells).
 constexpr unsigned CLOSED = 0x8000u;
 
+// Phase C's last part for one cell and layer: what leaves the cell through its edges (each edge's value F l_e cdt, rounded as
+// the grid-wide pass rounds it, in ascending edge order), and the limiter's factor.
+__device__ __forceinline__ double leaving(const double *F, uint4 w, const double lq[6], double cdt, unsigned pad) {
+  double out = 0;
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const unsigned v = slot_of(w, q);
+    if (v == pad) continue;                                    // a padded slot
+    const double x = F[v >> 1] * lq[q] * cdt;
+    if (!(v & 1u)) { if (x > 0) out += x; }
+    else if (!(x > 0)) out -= x;
+  }
+  return out;
+}
+
+// What flows out of a cell in one layer.
+__device__ __forceinline__ double outflow(const double *F, uint3 w, unsigned pad) {
+  double div = 0;
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const unsigned v = slot_of(w, q);
+    if (v != pad) div += slot_flux(F, v);
+  }
+  return div;
+}
+
+// The stage's end of a stack whose layers do not fit in shared memory together: phases C and D for d.lg layers at a time, one
+// exchange each, with the values of the register forms below. It walks the tile's edges instead of keeping them in registers
+// (mean: the edges' mean barotropic wind, in shared memory; their barotropic change in global memory), because state kept in
+// registers from group to group spilled. A step of one level-7 stack, grid-wide / groups with state in registers / this:
+// 6 mixed layers 1.056 / 1.103 / 0.987 ms, 8 mixed 1.789 / 1.857 / 1.715, 5 FP64 1.302 / 1.383 / 1.301, 8 FP64 1.618 /
+// 1.662 / 1.583; four level-6 stacks of 8 layers in one batch 1.595 -> 1.516 FP64, 1.770 -> 1.638 mixed.
+template <int NT, bool MIXED, bool WALL>
+__device__ __forceinline__ void end_in_groups(const StackDesc &d, int p, int st, unsigned *flags, unsigned turn, BatchStatus *status,
+                                              long long timeout_ns, bool skip, const int *eid, const int *cid, double *mean,
+                                              const int *cnt) {
+  const LayersDev &M = d.M;
+  const TileSetDev &T = d.tiles;
+  const int t = threadIdx.x, N = M.g.N, E = M.g.E, c0 = T.cell_off[p], e0 = T.edge_off[p];
+  const int nown = cnt[0], nc1 = cnt[1], eown = T.eown[p], ering = cnt[FAST_KMAX + 1];
+  const unsigned pad = 2u * (T.edge_off[p + 1] - e0);
+  const StageArgs a = stage_args(d, st);
+  const mixed::MStageArgs am = mixed::mstage_args(d, st);
+  double *F = mean + ering, *sc = F + (size_t)d.lg * ering;
+  bool finite = true;
+  for (int l0 = 0; l0 < d.L; l0 += d.lg) {
+    const int L = min(d.lg, d.L - l0);
+    if (l0 > 0) __syncthreads();                               // the layers before are done with F and sc
+    for (int e = t; e < ering; e += NT) {
+      const int2 x = T.eix[e0 + e];
+      const double m = mean[e];
+      if (MIXED) {
+        const double *ha = am.hs + (size_t)l0 * N + cid[x.y & 0xffff], *hb = am.hs + (size_t)l0 * N + cid[(unsigned)x.y >> 16];
+        const float *us = am.us + (size_t)l0 * E + x.x, ubs = M.ubs32[x.x];
+#pragma unroll 4
+        for (int l = 0; l < L; l++)
+          F[l * ering + e] = (0.5 * (ha[(size_t)l * N] + hb[(size_t)l * N])) * ((double)(us[(size_t)l * E] - ubs) + m);
+      } else {
+        const bool closed = WALL && M.wall && M.wall[x.x] == 0;
+        const double *he = M.hedge + (size_t)l0 * E + x.x, *us = a.us + (size_t)l0 * E + x.x, ubs = M.ubs[x.x];
+#pragma unroll 4
+        for (int l = 0; l < L; l++) {
+          const double h = he[(size_t)l * E];
+          F[l * ering + e] = closed ? 0.0 : h * (us[(size_t)l * E] - ubs) + h * m;
+        }
+      }
+    }
+    __syncthreads();
+    for (int c = t; c < nown; c += NT) {
+      const uint4 w = T.casc[c0 + c];
+      double lq[6];
+#pragma unroll
+      for (int q = 0; q < 6; q++) {
+        const unsigned v = slot_of(w, q);
+        lq[q] = v == pad ? 0.0 : T.el[e0 + (v >> 1)].x;
+      }
+      const double ar = T.aarea[c0 + c];
+      for (int l = 0; l < L; l++) {
+        const size_t o = (size_t)(l0 + l) * N + cid[c];
+        const double avail = a.h0[o] - M.floor_, out = leaving(F + l * ering, w, lq, a.cdt, pad);
+        const double cap = (avail > 0 ? avail : 0.0) * ar;
+        if (MIXED) {
+          const float s = out > cap ? __double2float_rz(cap / out) : 1.f;
+          sc[l * nc1 + c] = (double)s;
+          __stcg(M.scale32 + o, s);
+        } else {
+          const double s = out > cap ? cap / out : 1.0;
+          sc[l * nc1 + c] = s;
+          __stcg(M.scale + o, s);
+        }
+      }
+    }
+    if (!tile_exchange(T, p, flags, ++turn, status, timeout_ns, skip)) return;
+    for (int q = nown + t; q < nc1; q += NT)
+      for (int l = 0; l < L; l++) {
+        const size_t o = (size_t)(l0 + l) * N + cid[q];
+        sc[l * nc1 + q] = MIXED ? (double)__ldcg(M.scale32 + o) : __ldcg(M.scale + o);
+      }
+    __syncthreads();
+    for (int e = t; e < ering; e += NT) {
+      const int2 x = T.eix[e0 + e];
+      const int i = x.y & 0xffff, j = (unsigned)x.y >> 16;
+      const double le = MIXED ? M.g.le[x.x] : T.el[e0 + e].x;
+      const bool own = e < eown, closed = !MIXED && WALL && M.wall && M.wall[x.x] == 0;
+      const double dub = own && !MIXED ? M.ub[x.x] : 0.0;
+      const float dubf = own && MIXED ? M.dub[x.x] : 0.f;
+#pragma unroll 4
+      for (int l = 0; l < L; l++) {
+        const size_t o = (size_t)(l0 + l) * E + x.x;
+        double f = F[l * ering + e];
+        if (MIXED) {                                           // the FP32 flux and factor, their product in FP64
+          const float ff = (float)f;
+          f = (double)ff * sc[l * nc1 + (ff > 0.f ? i : j)] * le;
+        } else {
+          f *= sc[l * nc1 + (f > 0 ? i : j)];
+          f = f * le;
+        }
+        F[l * ering + e] = f;
+        if (!own) continue;
+        if (!MIXED) {
+          if (a.Fm) a.Fm[o] = f * a.dt;
+          a.un[o] = closed ? 0.0 : a.u0[o] + a.cdt * M.Tp[o] + dub;
+        } else if (am.un) {
+          if (am.Fm) am.Fm[o] = f * am.dt;
+          am.un[o] = am.u0[o] + __fma_rn(am.cdt, (double)M.Tp32[o], (double)dubf);
+        } else {
+          am.unf[o] = am.u0f[o] + __fmaf_rn((float)am.cdt, M.Tp32[o], dubf);
+        }
+      }
+    }
+    __syncthreads();
+    for (int c = t; c < nown; c += NT) {
+      const uint4 w = T.cedge[c0 + c];
+      const double ar = MIXED ? M.g.rA[cid[c]] : T.aarea[c0 + c];
+      for (int l = 0; l < L; l++) {
+        const size_t o = (size_t)(l0 + l) * N + cid[c];
+        const double h0 = a.h0[o], div = outflow(F + l * ering, make_uint3(w.x, w.y, w.z), pad);
+        const double h = MIXED ? __fma_rn(-(a.cdt * div), ar, h0) : h0 - (a.cdt * div) / ar;
+        a.hn[o] = h;
+        finite = finite && isfinite(h);
+      }
+    }
+  }
+  if (st == 2 && !finite && d.check) raise_status(status, ISW_ENOTFINITE);
+}
+
 template <int NT, int CAP, bool WALL>
 __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, unsigned *flags, BatchStatus *status,
                                           long long timeout_ns, bool skip, unsigned char *smem, const int *cnt) {
@@ -229,6 +375,17 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
       }
     }
   }
+  if (TILE_CAP[CAP].groups) {
+    double *mean = reinterpret_cast<double *>(work);
+#pragma unroll
+    for (int j = 0; j < AM; j++) {
+      const int e = t + j * NT;
+      if (e < ering) mean[e] = acc[j] * d.inv_n[st];
+      if (e < eown) M.ub[eid[e]] = ub[j] - M.ub0[eid[e]];
+    }
+    end_in_groups<NT, false, WALL>(d, p, st, flags, turn, status, timeout_ns, skip, eid, cid, mean, cnt);
+    return;
+  }
   // ---- phase C: the layer fluxes of the own cells' edges and the limiter factors of the own cells ----
   const StageArgs a = stage_args(d, st);
   const int L = d.L, N = M.g.N, E = M.g.E, nc1 = cnt[1];
@@ -262,7 +419,6 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
     }
   }
   __syncthreads();
-  // (the edge values a cell sums: F l_e cdt, rounded as the grid-wide pass rounds them)
 #pragma unroll
   for (int j = 0; j < CM; j++) {
     const int c = t + j * NT;
@@ -278,15 +434,7 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
       for (int l = 0; l < L; l++) {
         const size_t o = (size_t)l * N + cid[c];
         const double avail = a.h0[o] - M.floor_;
-        double out = 0;
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-          const unsigned v = slot_of(w, q);
-          if (v == 2u * ne) continue;                          // a padded slot
-          const double x = F[l * ering + (v >> 1)] * lq[q] * a.cdt;
-          if (!(v & 1u)) { if (x > 0) out += x; }
-          else if (!(x > 0)) out -= x;
-        }
+        const double out = leaving(F + l * ering, w, lq, a.cdt, 2u * ne);
         const double cap = (avail > 0 ? avail : 0.0) * ar;
         const double s = out > cap ? cap / out : 1.0;
         sc[l * nc1 + c] = s;
@@ -337,12 +485,7 @@ __device__ __forceinline__ void tile_fp64(const StackDesc &d, int p, int st, uns
       for (int l = 0; l < L; l++) {
         const size_t o = (size_t)l * N + cid[c];
         const double h0 = a.h0[o];
-        double div = 0;
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-          const unsigned v = slot_of(sl[j], q);
-          if (v != 2u * ne) div += slot_flux(F + l * ering, v);
-        }
+        const double div = outflow(F + l * ering, sl[j], 2u * ne);
         const double h = h0 - (a.cdt * div) / area[c];
         a.hn[o] = h;
         finite = finite && isfinite(h);
@@ -518,6 +661,17 @@ __device__ __forceinline__ void tile_mixed(const StackDesc &d, int p, int st, un
       }
     }
   }
+  if (TILE_CAP[CAP].groups) {
+    double *mean = reinterpret_cast<double *>(work);
+#pragma unroll
+    for (int j = 0; j < AM; j++) {
+      const int e = t + j * NT;
+      if (e < ering) mean[e] = __fma_rn(acc[j], d.inv_n[st], M.ub0[eid[e]]);
+      if (e < eown) M.dub[eid[e]] = dub[j];
+    }
+    end_in_groups<NT, true, false>(d, p, st, flags, turn, status, timeout_ns, skip, eid, cid, mean, cnt);
+    return;
+  }
   // ---- phase C ----
   const mixed::MStageArgs a = mixed::mstage_args(d, st);
   const int L = d.L, N = M.g.N, E = M.g.E, nc1 = cnt[1];
@@ -568,15 +722,7 @@ __device__ __forceinline__ void tile_mixed(const StackDesc &d, int p, int st, un
       for (int l = 0; l < L; l++) {
         const size_t o = (size_t)l * N + cid[c];
         const double avail = a.h0[o] - M.floor_;
-        double out = 0;
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-          const unsigned v = slot_of(w, q);
-          if (v == 2u * ne) continue;
-          const double x = F[l * ering + (v >> 1)] * lq[q] * a.cdt;
-          if (!(v & 1u)) { if (x > 0) out += x; }
-          else if (!(x > 0)) out -= x;
-        }
+        const double out = leaving(F + l * ering, w, lq, a.cdt, 2u * ne);
         const double cap = (avail > 0 ? avail : 0.0) * ar;
         const float s = out > cap ? __double2float_rz(cap / out) : 1.f;   // rounded toward zero
         sc[l * nc1 + c] = (double)s;
@@ -629,12 +775,7 @@ __device__ __forceinline__ void tile_mixed(const StackDesc &d, int p, int st, un
       for (int l = 0; l < L; l++) {
         const size_t o = (size_t)l * N + cid[c];
         const double h0 = a.h0[o];
-        double div = 0;
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-          const unsigned v = slot_of(sl[j], q);
-          if (v != 2u * ne) div += slot_flux(F + l * ering, v);
-        }
+        const double div = outflow(F + l * ering, sl[j], 2u * ne);
         const double h = __fma_rn(-(a.cdt * div), rAd, h0);
         a.hn[o] = h;
         finite = finite && isfinite(h);
@@ -673,8 +814,8 @@ Kernel kernel_for(int form) {
 }
 
 Kernel kernel_for(int bps, int cap, int form) {
-  if (bps == 2) return cap == 0 ? kernel_for<TILE_NT2, 0>(form) : kernel_for<TILE_NT2, 1>(form);
-  return cap == 0 ? kernel_for<TILE_NT1, 0>(form) : kernel_for<TILE_NT1, 1>(form);
+  if (bps == 2) return cap == 0 ? kernel_for<TILE_NT2, 0>(form) : cap == 1 ? kernel_for<TILE_NT2, 1>(form) : kernel_for<TILE_NT2, 2>(form);
+  return cap == 0 ? kernel_for<TILE_NT1, 0>(form) : cap == 1 ? kernel_for<TILE_NT1, 1>(form) : kernel_for<TILE_NT1, 2>(form);
 }
 
 }  // namespace

@@ -20,12 +20,15 @@ namespace isw {
 
 // What one tile may hold: thread t of a block of NT keeps the state of cells t, t + NT, ... and edges t, t + NT, ... in
 // registers (80 a thread), so a tile has at most C x NT cells, E x NT edges and A x NT edges of its own cells, whose
-// sub-step sums are kept. Two capacities, a kernel each: the small one keeps all of it in registers, the large one (which
-// lets a level-7 stack of 163,842 cells fill 148 SMs) spills some.
+// sub-step sums are kept. Two capacities: the small one keeps all of it in registers but for 4 bytes a thread (48 in the
+// mixed form), the large one (which lets a level-7 stack of 163,842 cells fill 148 SMs) spills some 100. The stage's end
+// holds the fluxes and limiter factors of all layers at once where they fit in shared memory; where they do not (level 7 on
+// 148 SMs: five FP64 layers, six mixed ones) the large capacity's other kernel takes them in groups of layers.
 struct TileCap {
   int C, E, A;
+  bool groups;
 };
-constexpr TileCap TILE_CAP[2] = {{2, 5, 3}, {2, 7, 5}};
+constexpr TileCap TILE_CAP[3] = {{2, 5, 3, false}, {2, 7, 5, false}, {2, 7, 5, true}};
 // Threads of a tile block when one or two tiles share an SM.
 constexpr int TILE_NT1 = 768, TILE_NT2 = 384;
 constexpr int TILE_FLAG_STRIDE = 8;            // a tile's exchange flag has a 32-byte sector of its own
@@ -43,14 +46,15 @@ struct TileSetHost {
   std::vector<int32_t> nbr_off, nbrs;          // per tile: the tiles it exchanges with (symmetric)
 };
 
-// Shared memory of a tile of nc cells (nc1 within one ring) and ne edges (ne0 of its own cells) of an L-layer stack: the
-// global ids (and the FP64 form's areas), then the fast loop's arrays, which the stage's end reuses. Fast loop, per edge
-// and cell: FP64 the flux l_e H_e ub, l_e H_e, (G, d_e); Y. Mixed the flux and its negative, (G, 1/d_e); Y. One flux more,
-// zero, for padded slots. Stage's end: the layer fluxes of the own cells' edges and the limiter factors, 8 bytes each.
-inline size_t tile_smem_bytes(size_t nc, size_t ne, size_t nc1, size_t ne0, size_t L, bool mixed) {
+// Shared memory of a tile of nc cells (nc1 within one ring) and ne edges (ne0 of its own cells) whose stage's end holds L
+// layers at once (groups: of more): the global ids (and the FP64 form's areas), then the fast loop's arrays, which the stage's
+// end reuses. Fast loop, per edge and cell: FP64 the flux l_e H_e ub, l_e H_e, (G, d_e); Y. Mixed the flux and its negative,
+// (G, 1/d_e); Y. One flux more, zero, for padded slots. Stage's end: the layer fluxes of the own cells' edges and the limiter
+// factors, 8 bytes each, in groups also the edges' mean barotropic wind.
+inline size_t tile_smem_bytes(size_t nc, size_t ne, size_t nc1, size_t ne0, size_t L, bool groups, bool mixed) {
   const size_t ids = (ne + nc + 1) / 2 * 8 + (mixed ? 0 : 8 * nc);
   const size_t loop = mixed ? (2 * (ne + 1) + 2 * ne + nc) * 4 : (4 * ne + 2 + nc) * 8;
-  const size_t end = 8 * L * (ne0 + nc1);
+  const size_t end = 8 * (L * (ne0 + nc1) + (groups ? ne0 : 0));
   return ids + 16 + (loop > end ? loop : end);   // (16: the loop's arrays start on a 16-byte boundary)
 }
 
