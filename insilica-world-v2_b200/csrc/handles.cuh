@@ -29,11 +29,15 @@ struct isw_layers {
   double nu4dt = 0;                 // nu4 dt of the last step (the exchange books the step's nabla^4 loss as heat)
   int version = 0;                  // bumped when an option is set: batches holding the stack rebuild its descriptor
   GraphEntry last_key{};            // option stacks: the arguments of the last direct step and the option version it saw
-  int last_version = -1;            // (a repeat of both steps through the private batch)
+  int last_version = -1;
+  int repeats = 0;                  // calls in a row that repeated the one before
+  int solo_wait = 1;                // repeats before the private batch is built for them, and the steps the last build served
+  int solo_steps = 0;
   bool percall = false;             // FP64: step with the per-call kernels instead of the private batch
   // the private one-stack batch (its step graph and tiles) that direct calls step through
   isw_batch *solo = nullptr;
   int solo_slot = -1;
+  int solo_version = -1;            // the option version its descriptor was last stepped with
   GraphEntry solo_key{};
   double *solo_Fm = nullptr;        // Fm when the caller passes none
 };

@@ -4,6 +4,7 @@
 // Launch sequence of one step: init, [lap cv, lap e] x 2 if nu4, then per stage: A, E, S, n x (eta, ubar), C, D; then
 // vmix if set. 21 + 2 sum_s n_s launches (95 at nfast = 20), against the reference's 35 + 2 sum_s n_s (+6 with nu4).
 // A direct call (stream not capturing) replays a cached CUDA graph of the whole step: one launch from the host.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <list>
@@ -492,8 +493,11 @@ void layers_step_solo(isw_layers *s, double *h, double *u, double *Fm, double dt
     s->solo_slot = slot;
     k = GraphEntry{h, u, Fm, nullptr, dt, nfast, nullptr};
   }
+  s->solo_version = s->version;
   ok(isw_batch_step(s->solo, st));
 }
+
+constexpr int SOLO_PAYS = 4, SOLO_WAIT_MAX = 64;
 
 void layers_step(isw_layers *s, double *h, double *u, double *Fm, double *theta, double dt, int nfast, cudaStream_t st) {
   if (!h || !u) fail(ISW_EINVAL, "layers.step: null h or u");
@@ -517,12 +521,23 @@ void layers_step(isw_layers *s, double *h, double *u, double *Fm, double *theta,
     const bool ready = s->solo && s->solo_slot >= 0 && same_call(s->solo_key, h, u, Fm ? Fm : s->solo_Fm, dt, nfast);
     bool solo = cs0 == cudaStreamCaptureStatusNone || ready;
     if (options) {
-      // option stacks: the private batch once a call repeats the one before it with no option set in between. Building it
-      // costs more than recording the per-call graph, of which eight are kept, so alternating arrays and options set before
-      // every step stay with the graphs. Never under a capture, nor while that batch would refuse to step for a non-finite
-      // thickness that a step without options left: option stacks are stepped whatever their thicknesses.
-      solo = cs0 == cudaStreamCaptureStatusNone && s->last_version == s->version && same_call(s->last_key, h, u, Fm, dt, nfast) &&
+      // option stacks: the private batch once calls repeat the one before them with no option set in between. Building it
+      // for other arguments or options takes 0.21 to 0.24 ms (B200, levels 4 and 6) and a step through it saves 0.12 to
+      // 0.14 over the per-call graph, of which eight are kept. So when a build served fewer than SOLO_PAYS steps before the
+      // next one, that one waits for twice the repeats: a caller that steps A, A, B, B, ... or sets an option every other
+      // step stays with the graphs after a few builds (level 6: 0.399 and 0.469 ms a call when every repeat built,
+      // 0.343 and 0.352 with the graphs alone, 0.311 and 0.353 now). Never under a capture, nor while that batch would refuse to step for a
+      // non-finite thickness that a step without options left: option stacks are stepped whatever their thicknesses.
+      const bool again = s->last_version == s->version && same_call(s->last_key, h, u, Fm, dt, nfast);
+      const bool built = ready && s->solo_version == s->version;
+      s->repeats = again ? s->repeats + 1 : 0;
+      solo = cs0 == cudaStreamCaptureStatusNone && again && (built || s->repeats >= s->solo_wait) &&
              !(s->solo && isw_batch_pending(s->solo));
+      if (solo && !built) {
+        if (s->solo_steps > 0) s->solo_wait = s->solo_steps < SOLO_PAYS ? std::min(2 * s->solo_wait, SOLO_WAIT_MAX) : 1;
+        s->solo_steps = 0;
+      }
+      if (solo) s->solo_steps++;
       s->last_key = GraphEntry{h, u, Fm, nullptr, dt, nfast, nullptr};
       s->last_version = s->version;
     }

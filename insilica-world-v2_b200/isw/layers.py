@@ -33,8 +33,8 @@ class Layers:
                  div_damp=DIV_DAMP, air=None, vmix=0.0, thin=2.0, wall=None, thin_wind=0.0, shelf=0.0, vmix_cd=0.0,
                  shelf_bed=False, batched=True, precision=None):
         """The reference's constructor (layers.py:36-37). batched (this core's): FP64 Boussinesq layers step through
-        a private one-stack batch (tiled fast loop, one graph; bit-identical results), with option branches from the first
-        call that repeats the one before it; False keeps the per-call kernels. precision (this core's): 'double' or 'mixed' for this object; None takes the grid's form
+        a private one-stack batch (tiled fast loop, one graph; bit-identical results), with option branches once
+        calls repeat the one before them; False keeps the per-call kernels. precision (this core's): 'double' or 'mixed' for this object; None takes the grid's form
         (the precision switch in force when the DeviceGrid was made)."""
         if precision not in (None, 'double', 'mixed'):
             raise ValueError(f'Layers: precision {precision!r}, want double or mixed')

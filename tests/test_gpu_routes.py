@@ -1,5 +1,5 @@
 """The step's routes for option stacks on a B200: through the private one-stack batch (its fast loop in tiles, walls
-included) from the first call that repeats the one before it, call by call otherwise; every mix equals the call-by-call
+included) once calls repeat the one before them, call by call otherwise; every mix equals the call-by-call
 kernels bit for bit."""
 from pathlib import Path
 
@@ -111,4 +111,37 @@ def test_timed_out_option_stack_is_refused(grid4):
         step(1)
     torch.cuda.synchronize()
     for x, y in zip(*states):
+        assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize('order', ['pairs', 'option'])
+def test_unpaid_builds_stop(grid4, order):
+    """Orders in which building the private batch does not pay (two sets of arrays in pairs of calls; an option set before
+    every other call) take no longer than the call-by-call kernels: host time per call in turns, the best of several. With
+    a build in every pair they took 1.5 to 2 times as long."""
+    import time
+    from isw.gpu import DeviceGrid
+    from isw.layers import Layers
+    z = golden('options_n4')
+    dg = DeviceGrid(grid4)
+    cores = [Layers(dg, 2, b=z['b'], gprime=[0.02], floor=1.0, batched=batched, wall=z['wall']) for batched in (True, False)]
+    sets = [[(T(z['h0']), T(z['u0']) * T(z['wall']), torch.zeros_like(T(z['u0']))) for _ in range(2)] for _ in cores]
+    tide = T(np.linspace(-0.3, 0.3, dg.N))
+
+    def calls(which, n):
+        for i in range(n):
+            if order == 'option' and i % 2 == 0:
+                cores[which].tide = tide if i % 4 == 0 else None
+            h, u, Fm = sets[which][i // 2 % 2 if order == 'pairs' else 0]
+            cores[which].step(h, u, float(z['dt']) / 4, 2, Fm)
+        torch.cuda.synchronize()
+    times = [[], []]
+    for turn in range(8):
+        for which in (0, 1):
+            t0 = time.perf_counter()
+            calls(which, 80)
+            if turn > 0:
+                times[which].append(time.perf_counter() - t0)
+    assert min(times[0]) < 1.25 * min(times[1]), times
+    for x, y in zip(*(s[0] + s[1] for s in sets)):
         assert torch.equal(x, y)
