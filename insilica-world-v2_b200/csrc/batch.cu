@@ -263,6 +263,7 @@ struct BatchSlot {
 struct FastGroup {
   int begin = 0, count = 0, form = 0, cap = 0;   // its tiles [begin, begin + count), their form, the kernel's capacity
   bool walls = false;                       // a stack of it has thin walls
+  int waited = -1;                          // a tile of it that another waits for (-1: every stack is one tile)
   size_t smem = 0;
 };
 
@@ -718,7 +719,7 @@ void rebuild(isw_batch *b) {
   const int ngroups = kbest > 0 ? 1 + *std::max_element(best.group.begin(), best.group.end()) : 0;
   std::vector<std::vector<TileRef>> grefs(ngroups);
   std::vector<size_t> gsmem(ngroups, 0);
-  std::vector<int> gform(ngroups, 0), gcap(ngroups, 0), gwalls(ngroups, 0);
+  std::vector<int> gform(ngroups, 0), gcap(ngroups, 0), gwalls(ngroups, 0), gwaited(ngroups, -1);
   std::vector<std::shared_ptr<TileCache>> used_tiles;
   std::vector<std::pair<size_t, int>> gfirst;     // per tiled stack in order: its group, its first tile within the group
   for (auto &sl : b->slots) {
@@ -768,6 +769,7 @@ void rebuild(isw_batch *b) {
       if (d.M.wall) gwalls[g] = 1;
       gcap[g] = std::max(gcap[g], d.lg < d.L ? 2 : tiles_cap(tc->host, best.K[q], best.bps));
       gfirst.emplace_back((size_t)g, (int)grefs[g].size());
+      if (best.P[q] > 1 && gwaited[g] < 0) gwaited[g] = (int)grefs[g].size();
       for (int p = 0; p < best.P[q]; p++) grefs[g].push_back(TileRef{s, p});
     }
     if (!d.tiled) any_untiled = 1;
@@ -855,6 +857,7 @@ void rebuild(isw_batch *b) {
     fg.form = gform[g];
     fg.cap = gcap[g];
     fg.walls = gwalls[g] != 0;
+    fg.waited = gwaited[g];
     refs.insert(refs.end(), grefs[g].begin(), grefs[g].end());
     b->groups.push_back(fg);
   }
@@ -1463,8 +1466,9 @@ int isw_batch_fault_test(isw_batch *b, long long timeout_ns, void *stream) {
     ISW_CUDA(cudaSetDevice(b->device));
     prepare(b);
     if (b->ntiles == 0) fail(ISW_EUNSUPPORTED, "batch.fault_test: no tiled stack in the batch");
+    if (b->groups[0].waited < 0) fail(ISW_EUNSUPPORTED, "batch.fault_test: stacks of one tile wait for no other");
     b->cur = b->d_desc;
-    launch_fast(b, (cudaStream_t)stream, 0, timeout_ns, 0);   // stage 0: it writes scratch only, every stage ends in an exchange
+    launch_fast(b, (cudaStream_t)stream, 0, timeout_ns, b->groups[0].waited);   // stage 0: it writes scratch only, every stage ends in an exchange
   });
 }
 

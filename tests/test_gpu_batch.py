@@ -185,6 +185,32 @@ def test_barrier_timeout_refuses_then_recovers(dev, grid4):
         assert torch.equal(x, y)
 
 
+def test_fault_test_needs_a_wait(dev, grid4):
+    """A stack of a single tile waits for no other: the failure test says so, and beside a stack of several tiles it takes
+    one of theirs."""
+    from isw import grid as G
+    from isw._lib import ISW_ETIMEOUT
+    from isw.batch import Batch
+    from isw.gpu import DeviceGrid
+    from isw.workload import Member, planet_grid
+    batch = Batch(0)
+    batch.config(layout='packed', blocks_per_sm=1)
+    a = Member(DeviceGrid(planet_grid(G.build(3, device='cpu'))), 4, nfast=20, batch=batch, kinds=('ocean',))
+    assert batch.info()['tiles'] == 1
+    with pytest.raises(NotImplementedError):
+        batch.fault_test(timeout_s=0.05)
+    assert batch.status() == 0
+    b = Member(DeviceGrid(planet_grid(grid4)), 4, nfast=20, batch=batch, kinds=('ocean',))
+    assert batch.info()['tiles'] > 2
+    batch.fault_test(timeout_s=0.05)
+    torch.cuda.synchronize()
+    assert batch.status(reset=True) == ISW_ETIMEOUT
+    batch.step()
+    torch.cuda.synchronize()
+    assert batch.status() == 0
+    assert all(bool(torch.isfinite(x).all()) for m in (a, b) for x in m.state())
+
+
 def test_status_reset_beside_steps_in_flight(dev, grid4):
     """Status resets from one thread while another steps the batch on a stream of its own: the tiles' exchange flags are
     left alone, no wait runs out, and the state equals an undisturbed run's bit for bit."""
