@@ -71,7 +71,7 @@ __device__ __forceinline__ void substep_chunk(const StackDesc &d, int st, int j,
 // buoyancy, the tide, the bottom's drag), instantiated only for batches holding such stacks, so that the plain
 // Boussinesq phases keep their register count.
 template <int PH, int LMAXK, bool EXT>
-__global__ void __launch_bounds__(THREADS) k_phase(const StackDesc *__restrict__ S, const Sched sc, int st, int j) {
+__global__ void __launch_bounds__(THREADS, phase_blocks_an_sm(PH, LMAXK, false)) k_phase(const StackDesc *__restrict__ S, const Sched sc, int st, int j) {
   Chunk ch{0, 0, 0};
   const int kind = phase_chunk<PH>(sc, blockIdx.x, ch);
   if (kind < 0) return;

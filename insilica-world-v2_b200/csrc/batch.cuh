@@ -180,6 +180,15 @@ __device__ __forceinline__ const StackDesc &stage_desc(const StackDesc *S, int s
 enum Phase { PH_INIT, PH_LAPE1, PH_LAPCV, PH_LAPE2, PH_A, PH_E, PH_S, PH_ETA, PH_UF, PH_CS, PH_D, PH_POST, PH_P2, PH_P3, PH_P4,
              PH_P1, PH_P2E, PH_P3E, PH_VMIX, PH_HF1, PH_VHEAT, PH_ONBED, PH_P1G, PH_P2G };
 
+// Blocks that must fit an SM (0: the compiler's choice), for the passes whose instances of six to eight layers otherwise take
+// registers for one block fewer. With one fewer, cold caches, 7 layers: P1 30.4 against 21.2 us and P4 32.1 against 22.6
+// (FP64, level 6), S 133.9 against 115.8 (mixed, level 7). Four mixed level-6 stacks of 7 layers and a tracer in one batch:
+// 1.348 ms a step with one fewer, 1.263 so.
+__host__ __device__ constexpr int phase_blocks_an_sm(int ph, int lmax, bool mixed) {
+  if (lmax < 8) return 0;
+  return ph == PH_P1 || (ph == PH_P4 && !mixed) ? 2 : ph == PH_S && mixed ? 3 : 0;
+}
+
 // Item i of the transport's edge passes: its edge, and its tracers [j0, j1).
 struct EdgeRow {
   int j0, j1, e;

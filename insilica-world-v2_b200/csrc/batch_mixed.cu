@@ -32,7 +32,7 @@ __device__ __forceinline__ void substep_chunk(const StackDesc &d, int st, int j,
 }
 
 template <int PH, int LMAXK>
-__global__ void __launch_bounds__(THREADS) k_phase_m(const StackDesc *__restrict__ S, const Sched sc, int st, int j) {
+__global__ void __launch_bounds__(THREADS, phase_blocks_an_sm(PH, LMAXK, true)) k_phase_m(const StackDesc *__restrict__ S, const Sched sc, int st, int j) {
   Chunk ch{0, 0, 0};
   const int kind = phase_chunk<PH>(sc, blockIdx.x, ch);
   if (kind < 0) return;

@@ -52,8 +52,9 @@ __global__ void __launch_bounds__(THREADS) k_stage_e(const LayersDev M, const St
   if (t < M.g.E) fp64::edge_hq<L>(M, a.hs, a.us, t);
 }
 
+// (two blocks an SM at eight layers too: level 6 83.4 -> 66.6 us)
 template <int L>
-__global__ void __launch_bounds__(THREADS) k_stage_s(const LayersDev M, const StageArgs a, const double *__restrict__ theta) {
+__global__ void __launch_bounds__(THREADS, L == 8 ? 2 : 0) k_stage_s(const LayersDev M, const StageArgs a, const double *__restrict__ theta) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < M.g.E) fp64::slow_edge<L>(M, a.cdt, t, theta);
 }

@@ -43,9 +43,10 @@ __global__ void __launch_bounds__(THREADS) k_mass(const GridDev g, int L, const 
     }                                                           \
   } while (0)
 
-// one thread per (tracer j, cell i), every layer of it
+// one thread per (tracer j, cell i), every layer of it (two blocks an SM at seven and eight layers too: 3 tracers of 7 layers
+// at level 7 by first order 130 -> 95 us; hf likewise at eight, where a third block, with 100 bytes of spills, ran slower)
 template <int L>
-__global__ void __launch_bounds__(THREADS) k_p1(const TransportDev T, const TrArgs a, int ntr, int order) {
+__global__ void __launch_bounds__(THREADS, L >= 7 ? 2 : 0) k_p1(const TransportDev T, const TrArgs a, int ntr, int order) {
   pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < T.g.N * ntr) fp64::tr_p1<L>(T, a, order, false, t / T.g.N, t % T.g.N);
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(THREADS) k_p1(const TransportDev T, const TrAr
 
 // one thread per (eg tracers, edge)
 template <int L>
-__global__ void __launch_bounds__(THREADS) k_hf(const TransportDev T, const TrArgs a, int ntr, int eg, int stage) {
+__global__ void __launch_bounds__(THREADS, L == 8 ? 2 : 0) k_hf(const TransportDev T, const TrArgs a, int ntr, int eg, int stage) {
   pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, j0 = t / T.g.E * eg;
   if (j0 < ntr) fp64::tr_hf_edge<L>(T, a, stage, j0, min(j0 + eg, ntr), t % T.g.E);
