@@ -212,11 +212,12 @@ int isw_batch_add_air(isw_batch *b, isw_layers *layers, isw_transport *tr, doubl
 int isw_batch_remove(isw_batch *b, int slot);
 int isw_batch_step(isw_batch *b, void *stream);
 /* Tuning (the autotuner's knobs; results are the same under every setting). The barotropic fast loop runs in
- * shared-memory tiles (tiles_enabled != 0, the default) exchanging every k sub-steps, k the largest up to tile_k (1..8,
- * default 8) whose tiles fit in shared memory, or as grid-wide passes. layout: 0 choose, 1 shared (one cooperative launch,
+ * on-chip tiles (tiles_enabled != 0, the default) exchanging every k sub-steps, k at most tile_k (1..8, default 8): the
+ * largest whose tiles fit a block, or with layout 0 the fastest of those by a model; or as grid-wide passes. layout: 0 choose, 1 shared (one cooperative launch,
  * every stack cut in proportion to its cells so the tiles fill the SMs), 2 packed (tiles of about tile_cells owned cells,
  * 64..4096, 0 = by blocks per SM; stacks packed into cooperative launches of at most SMs x blocks-per-SM tiles).
- * blocks_per_sm: 0 choose, 1 (1024-thread tiles) or 2 (512-thread tiles). */
+ * blocks_per_sm: 0 choose, 1 (768-thread tiles) or 2 (384-thread tiles). A block holds at most 1536 cells, the halo
+ * included (768 with two an SM): a stack whose tiles would be larger takes the grid-wide passes. */
 int isw_batch_config(isw_batch *b, int tiles_enabled, int tile_k, int layout, int tile_cells, int blocks_per_sm);
 /* How the untiled stacks run their grid-wide sub-steps. ISW_GRID_SPLIT (the default): two kernel launches per
  * sub-step, a cell pass and an edge pass. ISW_GRID_PERSISTENT: one cooperative launch per stage and precision form whose
@@ -248,7 +249,8 @@ int isw_batch_info(isw_batch *b, int *stacks, int *tiles, int *tile_k, long long
  * waits for the device and clears the word (restore the state first); steps in flight on other streams are unharmed. */
 int isw_batch_status(isw_batch *b, void *stream, int reset);
 /* Failure-detection test: the first stage's tile launch with a tile that never raises its flag, so its neighbours'
- * bounded wait runs out after timeout_ns (1 ms .. 2 s) and the status word becomes ISW_ETIMEOUT. Test use only. */
+ * bounded wait runs out after timeout_ns (1 ms .. 2 s) and the status word becomes ISW_ETIMEOUT; ISW_EUNSUPPORTED when
+ * no tile waits for another. Test use only. */
 int isw_batch_fault_test(isw_batch *b, long long timeout_ns, void *stream);
 
 /* Build the level-n mesh (N = 10 4^n + 2 cells) on the host: icosphere, Lloyd smoothing to 1e-11 rad (at most max_iters

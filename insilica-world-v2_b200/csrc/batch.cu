@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(THREADS, phase_blocks_an_sm(PH, LMAXK, false))
       if ((M.vmix != 0 || M.vmix_cd != 0) && d.L > 1) ISW_BATCH_L(d.L, LMAXK, fp64::vmix_edge<LL, EXT>(M, d.h, d.u, d.dt, i));
     } else {
       const EdgeRow r = edge_row(d, i);
-    ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
+      ISW_BATCH_L(d.L, LMAXK, fp64::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
     }
   } else if (PH == PH_P1 || PH == PH_P1G) {
     const CellRow r = cell_row(d, i);
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(THREADS) k_fast_grid(const StackDesc *__restri
         else fp64::bt_eta_cell_y(d.M, d.tau[st], j, i);
       }
     }
-    if (!grid_sync(bar, status, timeout_ns, 0)) return;
+    if (!grid_sync(bar, status, timeout_ns)) return;
     for (int c = blockIdx.x; c < sc.nuedge; c += gridDim.x) {
       const Chunk ch = sc.uedge[c];
       select(ch.s);
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(THREADS) k_fast_grid(const StackDesc *__restri
         }
       }
     }
-    if (!grid_sync(bar, status, timeout_ns, 0)) return;
+    if (!grid_sync(bar, status, timeout_ns)) return;
   }
 }
 
@@ -299,7 +299,7 @@ struct isw_batch {
   int any_ext = 0;                            // air or option stacks: the phase kernels with those branches
   int any_ob = 0;                             // a stack with the shelf's bed flags: their pass opens the step
   size_t fast_smem = 0;
-  int fast_bps = 2;                           // tile blocks per SM: 2 (256 threads each) or 1 (512 threads)
+  int fast_bps = 2;                           // tile blocks per SM: 2 (384 threads each) or 1 (768 threads)
   GridBarrier *bar = nullptr;
   unsigned *flags = nullptr;                  // the tiles' exchange flags, TILE_FLAG_STRIDE apart
   BatchStatus *status = nullptr;              // device status word (code + the mirror's device address)
@@ -535,9 +535,11 @@ bool tiles_form(const isw_batch *b, const BatchSlot &sl) {
 }
 
 // Modelled time (us) of a stack's tile launches in one step at exchange interval k <= the probe's: per stage a fixed part
-// (staging, the stage's end), per exchange its latency, per sub-step the edges the largest tile updates. The constants are
-// B200 timings of the kernel's phases at levels 6 and 7 (148 tiles of 553 and 1107 cells): staging and end 22 us, an
-// exchange 3.5 us, a sub-step 0.76 ns (FP64) or 0.40 ns (mixed) per edge and tile on the SM and at least 0.7 us.
+// (staging, the stage's end), per exchange its latency, per sub-step the edges the largest tile updates. It ranks tilings
+// against one another, not against the grid-wide sub-steps (Batch.autotune times both). The constants are B200 timings of
+// an earlier form of the kernel, 1,024 threads: staging and end 22 us for tiles of 553 cells (two or three layers; some 36
+// at 1,107), an exchange 3.5 us, a sub-step 0.76 ns (FP64) or 0.40 ns (mixed) per edge and tile on the SM and at least 0.7.
+// The present form's at 553 cells: 19 us, 2.4 to 3.0 us, 1.9 us a sub-step (FP64) or 1.1.
 double tiles_us(const TileSetHost &h, int k, int L, int nfast, bool mixed, int bps) {
   const double cs[3] = {1.0 / 3.0, 1.0 / 2.0, 1.0};
   const int lg = end_group(h, k, L, mixed, bps);

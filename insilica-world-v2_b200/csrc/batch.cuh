@@ -93,7 +93,7 @@ __device__ __forceinline__ long long globaltimer() {
 }
 
 // Block-wide grid barrier with a bounded wait. Returns false once any block has recorded a failure.
-__device__ inline bool grid_sync(GridBarrier *b, BatchStatus *status, long long timeout_ns, int skip_arrive) {
+__device__ inline bool grid_sync(GridBarrier *b, BatchStatus *status, long long timeout_ns) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -102,7 +102,7 @@ __device__ inline bool grid_sync(GridBarrier *b, BatchStatus *status, long long 
     cuda::atomic_ref<int, cuda::thread_scope_device> st(status->code);
     const unsigned g0 = gen.load(cuda::memory_order_acquire);
     __threadfence();
-    if (!skip_arrive && cnt.fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) {
+    if (cnt.fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) {
       cnt.store(0u, cuda::memory_order_relaxed);
       gen.fetch_add(1u, cuda::memory_order_release);
     } else {
@@ -185,6 +185,7 @@ enum Phase { PH_INIT, PH_LAPE1, PH_LAPCV, PH_LAPE2, PH_A, PH_E, PH_S, PH_ETA, PH
 // (FP64, level 6), S 133.9 against 115.8 (mixed, level 7). Four mixed level-6 stacks of 7 layers and a tracer in one batch:
 // 1.348 ms a step with one fewer, 1.263 so.
 __host__ __device__ constexpr int phase_blocks_an_sm(int ph, int lmax, bool mixed) {
+  if (lmax == 3 && ph == PH_P1 && mixed) return 4;             // (66 registers of its own accord)
   if (lmax < 8) return 0;
   return ph == PH_P1 || (ph == PH_P4 && !mixed) ? 2 : ph == PH_S && mixed ? 3 : 0;
 }

@@ -101,17 +101,15 @@ __global__ void __launch_bounds__(THREADS, phase_blocks_an_sm(PH, LMAXK, true)) 
       if ((M.vmix != 0 || M.vmix_cd != 0) && d.L > 1) ISW_BATCH_L(d.L, LMAXK, fp64::vmix_edge<LL, false>(M, d.h, d.u, d.dt, i));
     } else {
       const EdgeRow r = edge_row(d, i);
-    ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
+      ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 1, r.j0, r.j1, r.e));
     }
   } else if (PH == PH_P1) {
-    const CellRow r = cell_row(d, i);
-    ISW_BATCH_L(d.L, LMAXK, (mixed::tr_c1<LL, phase_tracers<PH>()>(d.T, d.tr, r.j0, r.n, r.c)));
+    ISW_BATCH_L(d.L, LMAXK, mixed::tr_c1<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
   } else if (PH == PH_P2E) {
     const EdgeRow r = edge_row(d, i);
     ISW_BATCH_L(d.L, LMAXK, mixed::tr_hf_edge<LL>(d.T, d.tr, 2, r.j0, r.j1, r.e));
   } else if (PH == PH_P2) {
-    const CellRow r = cell_row(d, i);
-    ISW_BATCH_L(d.L, LMAXK, (mixed::tr_c2<LL, phase_tracers<PH>()>(d.T, d.tr, r.j0, r.n, r.c)));
+    ISW_BATCH_L(d.L, LMAXK, mixed::tr_c2<LL>(d.T, d.tr, i / M.g.N, i % M.g.N));
   } else if (PH == PH_P3E) {
     const EdgeRow r = edge_row(d, i);
     ISW_BATCH_L(d.L, LMAXK, mixed::tr_a_edge<LL>(d.T, d.tr, r.j0, r.j1, r.e));
@@ -196,7 +194,7 @@ __global__ void __launch_bounds__(THREADS) k_fast_grid_m(const StackDesc *__rest
       const int i = ch.begin + (int)threadIdx.x;
       if (i < ch.end && j < d.n[st]) mixed::bt_eta_cell(d.M, (float)d.tau[st], j, d.n[st], i);
     }
-    if (!grid_sync(bar, status, timeout_ns, 0)) return;
+    if (!grid_sync(bar, status, timeout_ns)) return;
     for (int c = blockIdx.x; c < sc.nuedge; c += gridDim.x) {
       const Chunk ch = sc.uedge[c];
       select(ch.s);
@@ -206,7 +204,7 @@ __global__ void __launch_bounds__(THREADS) k_fast_grid_m(const StackDesc *__rest
         if (j == d.n[st] - 1) mixed::flux_edge(d.M, mixed::mstage_args(d, st), d.M.acc[i], i);
       }
     }
-    if (!grid_sync(bar, status, timeout_ns, 0)) return;
+    if (!grid_sync(bar, status, timeout_ns)) return;
   }
 }
 

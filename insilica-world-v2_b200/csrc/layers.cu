@@ -526,9 +526,9 @@ void layers_step(isw_layers *s, double *h, double *u, double *Fm, double *theta,
       // for other arguments or options takes 0.21 to 0.24 ms (B200, levels 4 and 6) and a step through it saves 0.12 to
       // 0.14 over the per-call graph, of which eight are kept. So when a build served fewer than SOLO_PAYS steps before the
       // next one, that one waits for twice the repeats: a caller that steps A, A, B, B, ... or sets an option every other
-      // step stays with the graphs after a few builds (level 6: 0.399 and 0.469 ms a call when every repeat built,
-      // 0.343 and 0.352 with the graphs alone, 0.311 and 0.353 now). Never under a capture, nor while that batch would refuse to step for a
-      // non-finite thickness that a step without options left: option stacks are stepped whatever their thicknesses.
+      // step stays with the graphs after a few builds (level 6, ms a call: 0.399 and 0.469 when every repeat built, 0.343
+      // and 0.352 with the graphs alone, 0.311 and 0.353 now). Never under a capture, nor while that batch would refuse to
+      // step for a non-finite thickness that a step without options left: option stacks are stepped whatever theirs are.
       const bool again = s->last_version == s->version && same_call(s->last_key, h, u, Fm, dt, nfast);
       const bool built = ready && s->solo_version == s->version;
       s->repeats = again ? s->repeats + 1 : 0;

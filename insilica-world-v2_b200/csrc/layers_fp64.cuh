@@ -570,9 +570,9 @@ __device__ __forceinline__ void bt_eta_cells_y(const LayersDev &M, double tau, i
 }
 
 // The layer fluxes of edge e once the stage's fast loop has finished (reference lay_flux, layers.cu:392-397), every
-// layer: F = h_e (u - ubar_s) + h_e acc / n, acc the sub-steps' sum of ubar. A batch with no tiled stack forms them in
-// the last grid-wide sub-step's edge pass, once per edge, and its phase C only sums them (scale_sum_cell); batches
-// with tiles recompute them in phase C (scale_cell: the tile kernel's tail has no spare parallelism for the gathers).
+// layer: F = h_e (u - ubar_s) + h_e acc / n, acc the sub-steps' sum of ubar. A batch's untiled stacks form them in the
+// last grid-wide sub-step's edge pass, once per edge, and their phase C only sums them (scale_sum_cell); the tile kernel
+// forms its tiled stacks' itself; the call-by-call path recomputes them in phase C (scale_cell).
 template <bool OPT = true>
 __device__ __forceinline__ void flux_edge(const LayersDev &M, const StageArgs &a, double acc, int e) {
   const GridDev &g = M.g;

@@ -155,25 +155,22 @@ __device__ __forceinline__ void tr_a_edge(const TransportDev &T, const TrArgs &a
     st_layers<L>(T.Af + fx(j, E, e, L), out);
   }
 }
-
-template <int L, int G>
-__device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, int j0, int n, int i) {
+// (one tracer a thread: two, as the FP64 passes take, left eight members 2.523 -> 2.535 ms a step)
+template <int L>
+__device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, int j, int i) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
   fp64::CellEdges c;
   fp64::load_edges(g, i, c);
-  double m1[L], mx[L], td[G][L], s[G][L], own[G][L];
+  double m1[L], mx[L], td[L], s[L], own[L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
     const double m0 = a.M0[om];
     m1[l] = m0;
     mx[l] = m0;
-#pragma unroll
-    for (int t = 0; t < G; t++) {
-      own[t][l] = t < n ? a.tr[j0 + t][om] : 0.0;
-      td[t][l] = s[t][l] = m0 * own[t][l];
-    }
+    own[l] = a.tr[j][om];
+    td[l] = s[l] = m0 * own[l];
   }
   const double frac = 1.0 / 3.0;
 #pragma unroll
@@ -181,62 +178,42 @@ __device__ __forceinline__ void tr_c1(const TransportDev &T, const TrArgs &a, in
     const int e = c.e[q];
     if (e >= 0) {
       const bool out = c.out[q];
-      double f[L];
+      double Av[L];
+      ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll
       for (int l = 0; l < L; l++) {
-        f[l] = a.Fm[(size_t)l * E + e];
-        const double m = frac * f[l];
-        if (out) { m1[l] -= f[l]; mx[l] -= m; }
-        else { m1[l] += f[l]; mx[l] += m; }
+        const double f = a.Fm[(size_t)l * E + e], pn = a.tr[j][(size_t)l * N + c.nb[q]];
+        const double fu = fp64::upwind_v(f, out ? own[l] : pn, out ? pn : own[l]);
+        const double hf = frac * Av[l], m = frac * f;
+        if (out) { m1[l] -= f; mx[l] -= m; td[l] -= fu; s[l] -= hf; }
+        else { m1[l] += f; mx[l] += m; td[l] += fu; s[l] += hf; }
       }
-#pragma unroll
-      for (int t = 0; t < G; t++)
-        if (t < n) {
-          double Av[L];
-          ld_layers<L>(T.A + fx(j0 + t, E, e, L), Av);
-#pragma unroll
-          for (int l = 0; l < L; l++) {
-            const double pn = a.tr[j0 + t][(size_t)l * N + c.nb[q]];
-            const double fu = fp64::upwind_v(f[l], out ? own[t][l] : pn, out ? pn : own[t][l]);
-            const double hf = frac * Av[l];
-            if (out) { td[t][l] -= fu; s[t][l] -= hf; }
-            else { td[t][l] += fu; s[t][l] += hf; }
-          }
-        }
     }
   }
+  double tdo[L];
+  float p1o[L];
 #pragma unroll
-  for (int t = 0; t < G; t++) {
-    if (t >= n) break;
-    const int j = j0 + t;
-    double tdo[L];
-    float p1o[L];
-#pragma unroll
-    for (int l = 0; l < L; l++) {
-      const size_t om = (size_t)l * N + i;
-      const double mm = m1[l];
-      if (j == 0) a.M1[om] = mm;
-      tdo[l] = td[t][l] / mm;
-      p1o[l] = (float)(s[t][l] / mx[l]);
-    }
-    st_layers<L>(T.td + fx(j, N, i, L), tdo);
-    st_layers<L>(T.p1f + fx(j, N, i, L), p1o);
+  for (int l = 0; l < L; l++) {
+    if (j == 0) a.M1[(size_t)l * N + i] = m1[l];
+    tdo[l] = td[l] / m1[l];
+    p1o[l] = (float)(s[l] / mx[l]);
   }
+  st_layers<L>(T.td + fx(j, N, i, L), tdo);
+  st_layers<L>(T.p1f + fx(j, N, i, L), p1o);
 }
 
-template <int L, int G>
-__device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, int j0, int n, int i) {
+template <int L>
+__device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, int j, int i) {
   const GridDev &g = T.g;
   const int N = g.N, E = g.E;
   fp64::CellEdges c;
   fp64::load_edges<false>(g, i, c);
-  double mx[L], s[G][L];
+  double mx[L], s[L];
 #pragma unroll
   for (int l = 0; l < L; l++) {
     const size_t om = (size_t)l * N + i;
     mx[l] = a.M0[om];
-#pragma unroll
-    for (int t = 0; t < G; t++) s[t][l] = t < n ? mx[l] * a.tr[j0 + t][om] : 0.0;
+    s[l] = mx[l] * a.tr[j][om];
   }
   const double frac = 1.0 / 2.0;
 #pragma unroll
@@ -244,32 +221,19 @@ __device__ __forceinline__ void tr_c2(const TransportDev &T, const TrArgs &a, in
     const int e = c.e[q];
     if (e >= 0) {
       const bool out = c.out[q];
+      double Av[L];
+      ld_layers<L>(T.A + fx(j, E, e, L), Av);
 #pragma unroll
       for (int l = 0; l < L; l++) {
-        const double m = frac * a.Fm[(size_t)l * E + e];
-        if (out) mx[l] -= m; else mx[l] += m;
+        const double m = frac * a.Fm[(size_t)l * E + e], hf = frac * Av[l];
+        if (out) { mx[l] -= m; s[l] -= hf; } else { mx[l] += m; s[l] += hf; }
       }
-#pragma unroll
-      for (int t = 0; t < G; t++)
-        if (t < n) {
-          double Av[L];
-          ld_layers<L>(T.A + fx(j0 + t, E, e, L), Av);
-#pragma unroll
-          for (int l = 0; l < L; l++) {
-            const double hf = frac * Av[l];
-            if (out) s[t][l] -= hf; else s[t][l] += hf;
-          }
-        }
     }
   }
+  float p2o[L];
 #pragma unroll
-  for (int t = 0; t < G; t++) {
-    if (t >= n) break;
-    float p2o[L];
-#pragma unroll
-    for (int l = 0; l < L; l++) p2o[l] = (float)(s[t][l] / mx[l]);
-    st_layers<L>(T.p2f + fx(j0 + t, N, i, L), p2o);
-  }
+  for (int l = 0; l < L; l++) p2o[l] = (float)(s[l] / mx[l]);
+  st_layers<L>(T.p2f + fx(j, N, i, L), p2o);
 }
 
 template <int L>

@@ -59,8 +59,9 @@ class Batch:
 
     def config(self, tiles=True, tile_k=8, layout='auto', tile_cells=0, blocks_per_sm=0, persistent=False, levels=None,
                grid=None):
-        """The fast loop in shared-memory tiles exchanging every k <= tile_k sub-steps (the largest that fits), or
-        grid-wide passes; layout 'shared' (one cooperative launch, tiles in proportion to each stack's cells), 'packed'
+        """The fast loop in on-chip tiles exchanging every k <= tile_k sub-steps (the largest that fits a block; with layout
+        'auto' the fastest of those by a model), or grid-wide passes; a stack whose tiles a block cannot hold (more than
+        1536 cells with their halo, 768 at two blocks per SM) takes the grid-wide passes; layout 'shared' (one cooperative launch, tiles in proportion to each stack's cells), 'packed'
         (tiles of about tile_cells owned cells, stacks packed into launches) or 'auto'; blocks_per_sm 1, 2 or 0 (auto).
         grid: how untiled stacks run their grid-wide sub-steps: 'split' (a cell launch and an edge launch per sub-step)
         or 'persistent' (one cooperative launch per stage, co-resident blocks meeting at a grid barrier after every pass);
@@ -156,8 +157,7 @@ class Batch:
             cur['levels'] = {lv: (start, 0, 0) for lv in levels}
             t_cur = times[key_of(best)]
             for lv in levels:
-                for opt in (('untiled', 0, 0), ('packed', 512, 3), ('packed', 1024, 3), ('packed', 1024, 4),
-                            ('packed', 2048, 4)):
+                for opt in (('untiled', 0, 0), ('packed', 512, 3), ('packed', 1024, 3), ('packed', 1024, 4)):
                     if cur['levels'][lv] == opt:
                         continue
                     cand = dict(cur, levels={**cur['levels'], lv: opt})
@@ -187,8 +187,8 @@ class Batch:
         _lib.check(_lib.isw_batch_flush(self._h, stream_of(self.device, stream)))
 
     def status(self, reset=False, stream=None):
-        """The device status word: 0, ISW_ETIMEOUT (5) after a tile's (or the grid barrier's) bounded wait ran out, or ISW_ENOTFINITE (6)
-        after a step left a NaN or Inf thickness. While it is set, step() raises IswError with that status; reset clears
+        """The device status word: 0, ISW_ETIMEOUT (5) after a tile's (or the grid barrier's) bounded wait ran out, or
+        ISW_ENOTFINITE (6) after a step left a NaN or Inf thickness. While it is set, step() raises IswError with that status; reset clears
         it (restore the state first)."""
         st = _lib.isw_batch_status(self._h, stream_of(self.device, stream), 1 if reset else 0)
         if st not in (_lib.ISW_OK, _lib.ISW_ETIMEOUT, _lib.ISW_ENOTFINITE):
@@ -196,5 +196,6 @@ class Batch:
         return st
 
     def fault_test(self, timeout_s=0.05, stream=None):
-        """One step in which a block never arrives at the first barrier: the others' bounded waits run out."""
+        """The first stage's tile launch with a tile that never raises its flag: its neighbours' bounded waits run out
+        (NotImplementedError when every stack is a single tile)."""
         _lib.check(_lib.isw_batch_fault_test(self._h, int(timeout_s * 1e9), stream_of(self.device, stream)))

@@ -1,6 +1,6 @@
 """The batched persistent step (isw.batch.Batch over the C ABI): each stack's result is bit-identical to stepping it
 alone, across stacks of different grids and layer counts in one launch; the golden vectors hold through it; and a
-grid barrier whose wait runs out reports ISW_ETIMEOUT to the host and leaves the context usable."""
+tile whose wait runs out reports ISW_ETIMEOUT to the host and leaves the context usable."""
 import numpy as np
 import pytest
 import torch
@@ -156,7 +156,7 @@ def test_batch_layout_per_level_equals_alone(dev, grid4, levels):
 
 
 def test_barrier_timeout_refuses_then_recovers(dev, grid4):
-    """A block that never arrives at a grid barrier: the others' bounded waits run out and the host reads ISW_ETIMEOUT.
+    """A tile that never raises its flag: its neighbours' bounded waits run out and the host reads ISW_ETIMEOUT.
     While the status is set the batch refuses to step (ISW_ETIMEOUT, nothing launched), so a caller that never polls
     cannot step on a half-updated state. Once reset, the SAME batch steps again and equals an untouched run of the same
     member bit for bit (the timed-out launch wrote only the fast loop's scratch, which every step rebuilds from h, u)."""
@@ -324,8 +324,7 @@ def test_tiled_fast_loop_equals_grid_wide(dev, grid4, k):
 def test_grid_wide_forms_equal(dev, grid4, precision):
     """The grid-wide sub-steps as two launches each (over wide chunks, several items a thread) give the persistent
     loop's result (item by item) bit for bit: members of different sub-step counts in one batch (nfast 20, 7 and 2, the
-    last with stages of one sub-step), and a grid-wide level beside a tiled one (the layer fluxes then formed in phase
-    C)."""
+    last with stages of one sub-step), and a grid-wide level beside a tiled one."""
     from isw import gpu
     from isw import grid as G
     from isw.batch import Batch
@@ -363,8 +362,8 @@ def test_grid_wide_forms_equal(dev, grid4, precision):
 
 
 def test_batch_of_both_forms(dev, grid4):
-    """One batch holding FP64 and mixed stacks (each phase one kernel per form, the mixed stacks' fast loop in tiles, the
-    FP64 stacks' as grid-wide sub-steps): every FP64 stack equals the same stack in an FP64-only batch bit for bit, and
+    """One batch holding FP64 and mixed stacks (each phase one kernel per form, the fast loop in tiles, one launch per form):
+    every FP64 stack equals the same stack in an FP64-only batch bit for bit, and
     every mixed stack equals the same stack in a mixed-only batch bit for bit."""
     from isw import gpu
     from isw.batch import Batch
