@@ -70,8 +70,8 @@ __device__ __forceinline__ void substep_chunk(const StackDesc &d, int st, int j,
 // EXT: the kernel also carries the air branch and the option branches (walls, the shelf and its bed flags, per-cell
 // buoyancy, the tide, the bottom's drag), instantiated only for batches holding such stacks, so that the plain
 // Boussinesq phases keep their register count.
-template <int PH, int LMAXK, bool EXT>
-__global__ void __launch_bounds__(THREADS, phase_blocks_an_sm(PH, LMAXK, false)) k_phase(const StackDesc *__restrict__ S, const Sched sc, int st, int j) {
+template <int PH, int LMAXK, bool EXT, int MINB = 0>
+__global__ void __launch_bounds__(THREADS, MINB) k_phase(const StackDesc *__restrict__ S, const Sched sc, int st, int j) {
   Chunk ch{0, 0, 0};
   const int kind = phase_chunk<PH>(sc, blockIdx.x, ch);
   if (kind < 0) return;
@@ -965,19 +965,21 @@ void launch_form(isw_batch *b, cudaStream_t st, int f, int stage, int j, bool pd
     return;
   }
   const size_t smem = PH == PH_S ? b->s_smem[0] : 0;
+  constexpr int MB = phase_blocks_an_sm(PH, 8, false);
+  const bool bounded = more_blocks(nb, MB);
   if (b->any_ext) {
     switch (b->lmax) {
       case 2: launch_kernel(k_phase<PH, 2, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
       case 3: launch_kernel(k_phase<PH, 3, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
       case 5: launch_kernel(k_phase<PH, 5, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
-      default: launch_kernel(k_phase<PH, 8, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+      default: launch_kernel(bounded ? k_phase<PH, 8, true, MB> : k_phase<PH, 8, true>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
     }
   } else {
     switch (b->lmax) {
       case 2: launch_kernel(k_phase<PH, 2, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
       case 3: launch_kernel(k_phase<PH, 3, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
       case 5: launch_kernel(k_phase<PH, 5, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
-      default: launch_kernel(k_phase<PH, 8, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
+      default: launch_kernel(bounded ? k_phase<PH, 8, false, MB> : k_phase<PH, 8, false>, nb, st, pdl, smem, b->cur, sc, stage, j); break;
     }
   }
 }

@@ -180,12 +180,14 @@ __device__ __forceinline__ const StackDesc &stage_desc(const StackDesc *S, int s
 enum Phase { PH_INIT, PH_LAPE1, PH_LAPCV, PH_LAPE2, PH_A, PH_E, PH_S, PH_ETA, PH_UF, PH_CS, PH_D, PH_POST, PH_P2, PH_P3, PH_P4,
              PH_P1, PH_P2E, PH_P3E, PH_VMIX, PH_HF1, PH_VHEAT, PH_ONBED, PH_P1G, PH_P2G };
 
-// Blocks that must fit an SM (0: the compiler's choice), for the passes whose instances of six to eight layers otherwise take
-// registers for one block fewer. With one fewer, cold caches, 7 layers: P1 30.4 against 21.2 us and P4 32.1 against 22.6
-// (FP64, level 6), S 133.9 against 115.8 (mixed, level 7). Four mixed level-6 stacks of 7 layers and a tracer in one batch:
-// 1.348 ms a step with one fewer, 1.263 so.
+// Blocks an SM that a launch bound asks of a pass (0: none), where the registers of its own accord leave one block fewer: the
+// instances of six to eight layers (and the mixed P1 of three, at 66). A launch takes the bounded kernel when it has more
+// blocks than fit without it. With one block fewer, cold caches, 7 layers: P1 30.4 against 21.2 us and P4 32.1 against 22.6
+// (FP64, level 6), S 133.9 against 115.8 (mixed, level 7); four mixed level-6 stacks of 7 layers and a tracer 1.348 ms a step
+// against 1.263. But where every block fits anyway the bound's spills cost: a mixed level-5 stack of 7 layers 0.228 ms
+// against 0.217.
 __host__ __device__ constexpr int phase_blocks_an_sm(int ph, int lmax, bool mixed) {
-  if (lmax == 3 && ph == PH_P1 && mixed) return 4;             // (66 registers of its own accord)
+  if (lmax == 3) return ph == PH_P1 && mixed ? 4 : 0;
   if (lmax < 8) return 0;
   return ph == PH_P1 || (ph == PH_P4 && !mixed) ? 2 : ph == PH_S && mixed ? 3 : 0;
 }

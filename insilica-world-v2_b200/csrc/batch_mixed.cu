@@ -31,8 +31,8 @@ __device__ __forceinline__ void substep_chunk(const StackDesc &d, int st, int j,
   }
 }
 
-template <int PH, int LMAXK>
-__global__ void __launch_bounds__(THREADS, phase_blocks_an_sm(PH, LMAXK, true)) k_phase_m(const StackDesc *__restrict__ S, const Sched sc, int st, int j) {
+template <int PH, int LMAXK, int MINB = 0>
+__global__ void __launch_bounds__(THREADS, MINB) k_phase_m(const StackDesc *__restrict__ S, const Sched sc, int st, int j) {
   Chunk ch{0, 0, 0};
   const int kind = phase_chunk<PH>(sc, blockIdx.x, ch);
   if (kind < 0) return;
@@ -126,11 +126,12 @@ __global__ void __launch_bounds__(THREADS, phase_blocks_an_sm(PH, LMAXK, true)) 
 template <int PH>
 void launch_m(int lmax, int nb, cudaStream_t st, bool pdl, size_t smem, const StackDesc *desc, const Sched &sc, int stage,
               int j) {
+  constexpr int MB3 = phase_blocks_an_sm(PH, 3, true), MB8 = phase_blocks_an_sm(PH, 8, true);
   switch (lmax) {
     case 2: launch_kernel(k_phase_m<PH, 2>, nb, st, pdl, smem, desc, sc, stage, j); break;
-    case 3: launch_kernel(k_phase_m<PH, 3>, nb, st, pdl, smem, desc, sc, stage, j); break;
+    case 3: launch_kernel(more_blocks(nb, MB3) ? k_phase_m<PH, 3, MB3> : k_phase_m<PH, 3>, nb, st, pdl, smem, desc, sc, stage, j); break;
     case 5: launch_kernel(k_phase_m<PH, 5>, nb, st, pdl, smem, desc, sc, stage, j); break;
-    default: launch_kernel(k_phase_m<PH, 8>, nb, st, pdl, smem, desc, sc, stage, j); break;
+    default: launch_kernel(more_blocks(nb, MB8) ? k_phase_m<PH, 8, MB8> : k_phase_m<PH, 8>, nb, st, pdl, smem, desc, sc, stage, j); break;
   }
 }
 
@@ -138,7 +139,7 @@ void launch_m(int lmax, int nb, cudaStream_t st, bool pdl, size_t smem, const St
 
 void slow_phase_smem_mixed(size_t bytes) {
   for (const void *fn : {(const void *)k_phase_m<PH_S, 2>, (const void *)k_phase_m<PH_S, 3>, (const void *)k_phase_m<PH_S, 5>,
-                         (const void *)k_phase_m<PH_S, 8>})
+                         (const void *)k_phase_m<PH_S, 8>, (const void *)k_phase_m<PH_S, 8, phase_blocks_an_sm(PH_S, 8, true)>})
     ISW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 

@@ -235,6 +235,9 @@ void launch_kernel(void (*kern)(KA...), int nb, cudaStream_t st, bool pdl, size_
   ISW_CUDA(cudaLaunchKernelEx(&cfg, kern, KA(args)...));
 }
 
+// Whether a launch of nb blocks has more of them than fit the GPU's 148 SMs at one block an SM fewer than `blocks`.
+inline bool more_blocks(int nb, int blocks) { return blocks > 0 && nb > 148 * (blocks - 1); }
+
 inline int blocks_for(long long n, int threads = THREADS) {
   long long b = (n + threads - 1) / threads;
   return (int)(b < 1 ? 1 : b);

@@ -52,11 +52,18 @@ __global__ void __launch_bounds__(THREADS) k_stage_e(const LayersDev M, const St
   if (t < M.g.E) fp64::edge_hq<L>(M, a.hs, a.us, t);
 }
 
-// (two blocks an SM at eight layers too: level 6 83.4 -> 66.6 us)
-template <int L>
-__global__ void __launch_bounds__(THREADS, L == 8 ? 2 : 0) k_stage_s(const LayersDev M, const StageArgs a, const double *__restrict__ theta) {
+// (a bound for two blocks an SM, MINB, is for eight layers where the launch has more blocks than SMs: level 6 83.4 -> 66.6 us)
+template <int L, int MINB = 0>
+__global__ void __launch_bounds__(THREADS, MINB) k_stage_s(const LayersDev M, const StageArgs a, const double *__restrict__ theta) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < M.g.E) fp64::slow_edge<L>(M, a.cdt, t, theta);
+}
+
+template <int L>
+void launch_stage_s(const LayersDev &M, const StageArgs &a, const double *theta, cudaStream_t st) {
+  const int nb = blocks_for(M.g.E);
+  if (L == 8 && more_blocks(nb, 2)) k_stage_s<L, L == 8 ? 2 : 0><<<nb, THREADS, 0, st>>>(M, a, theta);
+  else k_stage_s<L><<<nb, THREADS, 0, st>>>(M, a, theta);
 }
 
 // ---- air layers ----
@@ -296,7 +303,7 @@ void enqueue_step(isw_layers *s, double *h, double *u, double *Fm, double dt, in
     a.inv_n = 1.0 / a.n;
     ISW_DISPATCH_L(L, (k_stage_a<LL><<<blocks_for(N + NV), THREADS, 0, st>>>(M, a)));
     ISW_DISPATCH_L(L, (k_stage_e<LL><<<blocks_for(E), THREADS, 0, st>>>(M, a)));
-    ISW_DISPATCH_L(L, (k_stage_s<LL><<<blocks_for(E), THREADS, 0, st>>>(M, a, nullptr)));
+    ISW_DISPATCH_L(L, launch_stage_s<LL>(M, a, nullptr, st));
     for (int j = 0; j < a.n; j++) {
       k_bt_eta<<<blocks_for(N), THREADS, 0, st>>>(M, a.tau);
       k_bt_u<<<blocks_for(E), THREADS, 0, st>>>(M, a.tau);
@@ -343,7 +350,7 @@ void enqueue_step_air(isw_layers *s, double *h, double *u, double *Fm, double *t
     a.inv_n = 1.0 / a.n;
     ISW_DISPATCH_L(L, (k_air_a<LL><<<blocks_for(N + NV), THREADS, 0, st>>>(M, a, theta)));
     ISW_DISPATCH_L(L, (k_air_e<LL><<<blocks_for(E), THREADS, 0, st>>>(M, a)));
-    ISW_DISPATCH_L(L, (k_stage_s<LL><<<blocks_for(E), THREADS, 0, st>>>(M, a, theta)));
+    ISW_DISPATCH_L(L, launch_stage_s<LL>(M, a, theta, st));
     for (int j = 0; j < a.n; j++) {
       ISW_DISPATCH_L(L, (k_af_muphi<LL><<<blocks_for(N), THREADS, 0, st>>>(M, a.tau)));
       ISW_DISPATCH_L(L, (k_af_u<LL><<<blocks_for(E), THREADS, 0, st>>>(M, a.tau)));

@@ -43,10 +43,11 @@ __global__ void __launch_bounds__(THREADS) k_mass(const GridDev g, int L, const 
     }                                                           \
   } while (0)
 
-// one thread per (tracer j, cell i), every layer of it (two blocks an SM at seven and eight layers too: 3 tracers of 7 layers
-// at level 7 by first order 130 -> 95 us; hf likewise at eight, where a third block, with 100 bytes of spills, ran slower)
-template <int L>
-__global__ void __launch_bounds__(THREADS, L >= 7 ? 2 : 0) k_p1(const TransportDev T, const TrArgs a, int ntr, int order) {
+// one thread per (tracer j, cell i), every layer of it (a bound for two blocks an SM, MINB, is for seven and eight layers
+// where the launch has more blocks than SMs: 3 tracers of 7 layers at level 7 by first order 130 -> 95 us; hf keeps two at
+// eight without spills, and ran slower with three and 100 bytes of them)
+template <int L, int MINB = 0>
+__global__ void __launch_bounds__(THREADS, MINB) k_p1(const TransportDev T, const TrArgs a, int ntr, int order) {
   pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < T.g.N * ntr) fp64::tr_p1<L>(T, a, order, false, t / T.g.N, t % T.g.N);
@@ -209,7 +210,7 @@ int isw_transport_step_many(isw_transport *t, const double *M0, const double *M1
     // the first kernel takes plain stream order, the others are programmatic dependents of the one before (8 tracers of 5
     // layers at level 6: 345 -> 334 us)
     if (order == 1) {
-      ISW_TR_L(t->L, launch_kernel(k_p1<LL>, nb, st, false, 0, t->d, a, ntr, order));
+      ISW_TR_L(t->L, launch_kernel(LL >= 7 && more_blocks(nb, 2) ? k_p1<LL, LL >= 7 ? 2 : 0> : k_p1<LL>, nb, st, false, 0, t->d, a, ntr, order));
       launch_kernel(k_td_out, blocks_for((long long)t->d.g.N * a.rows), st, true, 0, t->d, a);
     } else {
       const int cg = fp64::cell_tracers((long long)t->d.g.N * ntr, t->L);
