@@ -102,3 +102,77 @@ def test_batched_step_layer_counts(dev, grid4, oracle_lib, L, tiles):
     for name, a, ref in (('h', h, oh), ('u', u, ou), ('Fm', Fm, oF), ('M', M, oM), ('tr0', gpsi[0], psi[0]),
                          ('tr1', gpsi[1], psi[1])):
         assert np.array_equal(a.cpu().numpy(), ref), name
+
+
+def _stack(dg, L, seed, T):
+    rng = np.random.default_rng(seed)
+    N, E = dg.host.N, dg.host.E
+    dev = 'cuda:0'
+    h = _T(300.0 + 10.0 * rng.random((L, N)), dev)
+    u = _T(0.5 * (rng.random((L, E)) - 0.5), dev)
+    M = (h * _T(np.asarray(dg.host.areaCell)[None], dev)).contiguous()
+    return h, u, torch.zeros_like(u), M, torch.zeros_like(M), [_T(rng.random((L, N)), dev) for _ in range(T)]
+
+
+@pytest.mark.parametrize('L', [7, 8])
+@pytest.mark.parametrize('form', ['double', 'mixed'])
+def test_many_blocks_equal_few(dev, grid4, form, L):
+    """A launch with more blocks than fit the SMs takes the passes' instances with a launch bound (batched P1 and P4, the
+    mixed S, the per-call P1): ten stacks of 16 tracers in one batch equal one of them alone with its tracers eight at a
+    time, and 16 tracers by first order equal two calls of eight, bit for bit."""
+    from isw import gpu, transport
+    from isw.batch import Batch
+    from isw.layers import Layers
+    dg = gpu.DeviceGrid(grid4)
+    kw = dict(gprime=[0.05] * (L - 1), floor=1.0, precision=form)
+
+    def run(stacks, T, first):
+        b, keep = Batch(0), []
+        for q in range(stacks):
+            core, tr = Layers(dg, L, **kw), transport.Transport(dg, layers=L, tracers=T, precision=form)
+            h, u, Fm, M, M1, ps = _stack(dg, L, 5, 16)
+            ps = ps[first:first + T]
+            b.add(core, h, u, Fm, tr=tr, M=M, M1=M1, tracers=ps, dt=600.0, nfast=3)
+            keep.append((core, tr, h, u, Fm, M, M1, ps))
+        b.step()
+        b.step()
+        torch.cuda.synchronize()
+        assert b.status() == 0
+        return keep[-1]
+    many, one, two = run(10, 16, 0), run(1, 8, 0), run(1, 8, 8)
+    for a, x, y in zip(many[2:6], one[2:6], two[2:6]):
+        assert torch.equal(a, x) and torch.equal(a, y)
+    assert all(torch.equal(a, x) for a, x in zip(many[7], one[7] + two[7]))
+    h, u, Fm, M, M1, ps = _stack(dg, L, 6, 16)
+    tr = transport.Transport(dg, layers=L, tracers=16, precision=form)
+    Fm = 1e-4 * float(M.min()) * u
+    tr.mass_after(M, Fm, M1)
+    apart = [p.clone() for p in ps]
+    tr.step_many(M, M1, Fm, ps, 1)
+    tr.step_many(M, M1, Fm, apart[:8], 1)
+    tr.step_many(M, M1, Fm, apart[8:], 1)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, x) for a, x in zip(ps, apart))
+
+
+def test_eight_layers_call_by_call_at_level6(dev):
+    """Eight layers call by call on the 122,880 edges of level 6 (the slow tendency's instance with a launch bound) equal the
+    batched step bit for bit."""
+    from isw import gpu
+    from isw import grid as G
+    from isw.batch import Batch
+    from isw.layers import Layers
+    from isw.workload import planet_grid
+    dg = gpu.DeviceGrid(planet_grid(G.build(6, device=0)))
+    kw = dict(gprime=[0.05] * 7, floor=1.0, precision='double')
+    h, u, Fm, *_ = _stack(dg, 8, 7, 0)
+    h2, u2, Fm2 = h.clone(), u.clone(), Fm.clone()
+    core, direct, b = Layers(dg, 8, **kw), Layers(dg, 8, batched=False, **kw), Batch(0)
+    b.add(core, h, u, Fm, dt=100.0, nfast=3)
+    for _ in range(2):
+        b.step()
+        direct.step(h2, u2, 100.0, 3, Fm2)
+    torch.cuda.synchronize()
+    assert b.status() == 0
+    for x, y in ((h, h2), (u, u2), (Fm, Fm2)):
+        assert torch.equal(x, y)
