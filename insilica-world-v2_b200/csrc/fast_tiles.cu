@@ -85,8 +85,8 @@ __device__ __forceinline__ float slot_flux(const float *fl, unsigned v) { return
 // Bit 15 of an edge's local cells: a thin wall closes it (tiles have at most 32000 cells).
 constexpr unsigned CLOSED = 0x8000u;
 
-// Phase C's last part for one cell and layer: what leaves the cell through its edges (each edge's value F l_e cdt, rounded as
-// the grid-wide pass rounds it, in ascending edge order), and the limiter's factor.
+// What leaves a cell through its edges in one layer, for the limiter: each edge's value F l_e cdt, rounded as the grid-wide
+// pass rounds it, in ascending edge order.
 __device__ __forceinline__ double leaving(const double *F, uint4 w, const double lq[6], double cdt, unsigned pad) {
   double out = 0;
 #pragma unroll
@@ -100,7 +100,7 @@ __device__ __forceinline__ double leaving(const double *F, uint4 w, const double
   return out;
 }
 
-// What flows out of a cell in one layer.
+// The divergence of a cell's limited fluxes in one layer.
 __device__ __forceinline__ double outflow(const double *F, uint3 w, unsigned pad) {
   double div = 0;
 #pragma unroll
